@@ -4,11 +4,9 @@
 // x * 2^256 mod p, always fully reduced to [0, p) at the boundary of every operation, so
 // results are word-for-word the values the reference's host code produces
 // (src/cuda/ff.cpp montmult_h / addm_h / subm_h, same layout as src/cuda/types.h
-// NWORDS_256BIT).  Products are CIOS Montgomery multiplications on 32x32->64 wide
-// products folded by add-with-carry chains; BN254 moduli are below 2^254, so the CIOS
-// accumulator never needs a tenth limb and a single conditional subtraction finishes
-// every product.  Units that call products out of line (the G1 MSM) compute the same
-// Montgomery product in radix 2^52 on the FP64 pipe instead (namespace dp52).
+// NWORDS_256BIT).  Products are Montgomery products on 32x32->64 multiply-adds with carry,
+// one row of a*b and one of m*p per limb of b; BN254 moduli are below 2^254, so the running
+// value fits nine limbs and a single conditional subtraction finishes every product.
 #pragma once
 #include <cstdint>
 
@@ -27,12 +25,6 @@ struct ModQ {  // base field q (the reference's MOD_GROUP, pidx 0)
                             R24 = 0x0a417ff6u, R25 = 0x47ab1effu, R26 = 0xcab8351fu, R27 = 0x06d89f71u;
   static constexpr uint32_t R30 = 0xda1530dfu, R31 = 0xb1cd6dafu, R32 = 0xa7283db6u, R33 = 0x62f210e6u,
                             R34 = 0x0ada0afbu, R35 = 0xef7f0b0cu, R36 = 0x2d592544u, R37 = 0x20fd6e90u;
-  // q in radix 2^52 and -q^-1 mod 2^52 (FP64-pipe product)
-  static CSB_DEV double L52(int i) {
-    return i == 0 ? 154029749239111.0 : i == 1 ? 2558044347618242.0 : i == 2 ? 423691504025962.0
-         : i == 3 ? 2817616741948264.0 : 53207371014449.0;
-  }
-  static constexpr double NP52 = 571208714576777.0;
 };
 struct ModR {  // scalar field r (the reference's MOD_FIELD, pidx 1)
   static constexpr uint32_t P0 = 0xf0000001u, P1 = 0x43e1f593u, P2 = 0x79b97091u, P3 = 0x2833e848u,
@@ -44,114 +36,7 @@ struct ModR {  // scalar field r (the reference's MOD_FIELD, pidx 1)
                             R24 = 0x53bb8085u, R25 = 0x8c49833du, R26 = 0x7f4e44a5u, R27 = 0x0216d0b1u;
   static constexpr uint32_t R30 = 0xb4bf0040u, R31 = 0x5e94d8e1u, R32 = 0x1cfbb6b8u, R33 = 0x2a489cbeu,
                             R34 = 0xa19fcfedu, R35 = 0x893cc664u, R36 = 0x7fcc657cu, R37 = 0x0cf8594bu;
-  static CSB_DEV double L52(int i) {
-    return i == 0 ? 551490712240129.0 : i == 1 ? 1275002230477886.0 : i == 2 ? 423691496731624.0
-         : i == 3 ? 2817616741948264.0 : 53207371014449.0;
-  }
-  static constexpr double NP52 = 551490712240127.0;
 };
-
-// ------------------------------------------------- products on the FP64 pipe ----------
-// Montgomery product in radix 2^52 (Emmart, Zheng and Weems, "Faster modular
-// exponentiation using double precision floating point arithmetic on the GPU", ARITH
-// 2018): limbs are exact integers held in doubles; a 52x52-bit product x*y < 2^104 splits
-// exactly into its high and low 52 bits with two round-toward-zero FMAs,
-//   h = fma_rz(x, y, 2^104)            = 2^104 + H 2^52   (bits of h: exponent | H)
-//   l = fma_rz(x, y, 2^104 + 2^52 - h) = 2^52 + L         (bits of l: exponent | L),
-// and the raw bit patterns are summed per column in 64-bit integers, the exponent bits
-// taken off in bulk by the column's starting value.  The multiplies run on the FP64 pipe
-// and the column sums on the integer ALU, which a 32-bit CIOS leaves saturated by its
-// add-with-carry chains (B200: 56 vs 46 G lazy products/s).
-// The 8x32-bit operands are re-cut into five 52-bit limbs, one of them shifted left by 4:
-// REDC in radix 2^52 divides by 2^260, so the result is a*b*2^-256 mod p, the same
-// Montgomery product as the 32-bit CIOS.  For a, b < 2p it is below
-// 16 a b / 2^260 + p < 2p (BN254: 64 p / 2^260 < 0.77), a lazily reduced value.
-#ifndef CSB_DP52
-#define CSB_DP52 1
-#endif
-namespace dp52 {
-constexpr uint64_t kMask = 0x000FFFFFFFFFFFFFull;
-constexpr uint64_t kBitsLo = 0x4330000000000000ull;  // bits of 2^52
-constexpr uint64_t kBitsHi = 0x4670000000000000ull;  // bits of 2^104
-// x*y into the column pair (lo: bits 0..51 of the product, hi: bits 52..103)
-CSB_DEV void acc_prod(double x, double y, uint64_t& lo, uint64_t& hi) {
-  const double h = __fma_rz(x, y, 0x1p104);
-  const double l = __fma_rz(x, y, 0x1.0000000000001p104 - h);
-  lo += (uint64_t)__double_as_longlong(l);
-  hi += (uint64_t)__double_as_longlong(h);
-}
-// products landing in column k of a 5x5 schoolbook product
-__host__ __device__ constexpr int terms(int k) { return (k < 0 || k > 8) ? 0 : (k < 4 ? k + 1 : 9 - k); }
-// column k starts at minus the exponent bits of its terms: a*b and m*p each put terms(k)
-// low halves and terms(k-1) high halves into it
-__host__ __device__ constexpr uint64_t col_start(int k) {
-  return (uint64_t)0 - (uint64_t)(2 * terms(k)) * kBitsLo - (uint64_t)(2 * terms(k - 1)) * kBitsHi;
-}
-// integer v < 2^52 as a double
-CSB_DEV double to_dbl(uint64_t v) { return __longlong_as_double((long long)(v | kBitsLo)) - 0x1p52; }
-CSB_DEV void words(const uint32_t (&x)[8], uint64_t (&w)[4]) {
-#pragma unroll
-  for (int i = 0; i < 4; i++) w[i] = x[2 * i] | (uint64_t)x[2 * i + 1] << 32;
-}
-// x = sum l_i 2^(52 i)
-CSB_DEV void cut(const uint32_t (&x)[8], double (&l)[5]) {
-  uint64_t w[4];
-  words(x, w);
-  l[0] = to_dbl(w[0] & kMask);
-  l[1] = to_dbl(((w[0] >> 52) | (w[1] << 12)) & kMask);
-  l[2] = to_dbl(((w[1] >> 40) | (w[2] << 24)) & kMask);
-  l[3] = to_dbl(((w[2] >> 28) | (w[3] << 36)) & kMask);
-  l[4] = to_dbl(w[3] >> 16);
-}
-// 16 x = sum l_i 2^(52 i)
-CSB_DEV void cut16(const uint32_t (&x)[8], double (&l)[5]) {
-  uint64_t w[4];
-  words(x, w);
-  l[0] = to_dbl((w[0] << 4) & kMask);
-  l[1] = to_dbl(((w[0] >> 48) | (w[1] << 16)) & kMask);
-  l[2] = to_dbl(((w[1] >> 36) | (w[2] << 28)) & kMask);
-  l[3] = to_dbl(((w[2] >> 24) | (w[3] << 40)) & kMask);
-  l[4] = to_dbl(w[3] >> 12);
-}
-// a*b*2^-256 mod p, lazily reduced (< 2p for a, b < 2p)
-template <class M>
-CSB_DEV void mont(const uint32_t (&x)[8], const uint32_t (&y)[8], uint32_t (&out)[8]) {
-  double a[5], b[5];
-  cut16(x, a);
-  cut(y, b);
-  uint64_t c[10];
-#pragma unroll
-  for (int k = 0; k < 10; k++) c[k] = col_start(k);
-#pragma unroll
-  for (int i = 0; i < 5; i++)
-#pragma unroll
-    for (int j = 0; j < 5; j++) acc_prod(a[i], b[j], c[i + j], c[i + j + 1]);
-#pragma unroll
-  for (int k = 0; k < 5; k++) {
-    if (k > 0) c[k] += c[k - 1] >> 52;  // column k-1 is complete (and 0 mod 2^52)
-    // m = (c_k mod 2^52) * (-p^-1) mod 2^52: the low half of one more split product
-    const double t = to_dbl(c[k] & kMask);
-    const double h = __fma_rz(t, M::NP52, 0x1p104);
-    const double m = __fma_rz(t, M::NP52, 0x1.0000000000001p104 - h) - 0x1p52;
-#pragma unroll
-    for (int j = 0; j < 5; j++) acc_prod(m, M::L52(j), c[k + j], c[k + j + 1]);
-  }
-  uint64_t r[5];
-  uint64_t carry = c[4] >> 52;
-#pragma unroll
-  for (int j = 0; j < 5; j++) {
-    const uint64_t v = c[5 + j] + carry;
-    carry = v >> 52;
-    r[j] = j < 4 ? (v & kMask) : v;
-  }
-  const uint64_t w0 = r[0] | (r[1] << 52), w1 = (r[1] >> 12) | (r[2] << 40);
-  const uint64_t w2 = (r[2] >> 24) | (r[3] << 28), w3 = (r[3] >> 36) | (r[4] << 16);
-  out[0] = (uint32_t)w0; out[1] = (uint32_t)(w0 >> 32);
-  out[2] = (uint32_t)w1; out[3] = (uint32_t)(w1 >> 32);
-  out[4] = (uint32_t)w2; out[5] = (uint32_t)(w2 >> 32);
-  out[6] = (uint32_t)w3; out[7] = (uint32_t)(w3 >> 32);
-}
-}  // namespace dp52
 
 // ------------------------------------------------------------ carry-chain helpers ----
 // Each helper is one PTX instruction; `volatile` keeps the carry flag sequence in
@@ -163,36 +48,73 @@ CSB_DEV void mont(const uint32_t (&x)[8], const uint32_t (&y)[8], uint32_t (&out
 #define SUBC_CC(d, a, b)    asm volatile("subc.cc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 #define SUBC(d, a, b)       asm volatile("subc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 
-// t[0..8] += a[0..7] * b using 32x32->64 wide products (IMAD.WIDE): the even-index
-// products a0b, a2b, a4b, a6b tile limbs 0..7 without overlap and the odd ones tile
-// limbs 1..8, so each half is a ready 8-limb addend; two add.cc chains fold them in.
-// Requires the true sum to fit in 9 limbs.
-CSB_DEV void row_mad_wide(uint32_t (&t)[9], const uint32_t (&a)[8], uint32_t b) {
-  asm volatile(
-      "{\n\t.reg .b64 p;\n\t.reg .u32 lo, hi;\n\t"
-      // even products: limbs 0..7, carry into t8
-      "mul.wide.u32 p, %9, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "add.cc.u32 %0, %0, lo;\n\taddc.cc.u32 %1, %1, hi;\n\t"
-      "mul.wide.u32 p, %11, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %2, %2, lo;\n\taddc.cc.u32 %3, %3, hi;\n\t"
-      "mul.wide.u32 p, %13, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %4, %4, lo;\n\taddc.cc.u32 %5, %5, hi;\n\t"
-      "mul.wide.u32 p, %15, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %6, %6, lo;\n\taddc.cc.u32 %7, %7, hi;\n\t"
-      "addc.u32 %8, %8, 0;\n\t"
-      // odd products: limbs 1..8
-      "mul.wide.u32 p, %10, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "add.cc.u32 %1, %1, lo;\n\taddc.cc.u32 %2, %2, hi;\n\t"
-      "mul.wide.u32 p, %12, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %3, %3, lo;\n\taddc.cc.u32 %4, %4, hi;\n\t"
-      "mul.wide.u32 p, %14, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %5, %5, lo;\n\taddc.cc.u32 %6, %6, hi;\n\t"
-      "mul.wide.u32 p, %16, %17;\n\tmov.b64 {lo, hi}, p;\n\t"
-      "addc.cc.u32 %7, %7, lo;\n\taddc.u32 %8, %8, hi;\n\t}"
-      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]),
-        "+r"(t[7]), "+r"(t[8])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]),
-        "r"(b));
+// Montgomery products accumulate in two sets of columns: e holds columns 0..7 as the 64-bit
+// pairs (0,1) (2,3) (4,5) (6,7), o columns 1..8 as (1,2) (3,4) (5,6) (7,8), and the value is
+// e + 2^32 o.  A limb's products with the even limbs of the other operand tile e's pairs and
+// those with its odd limbs tile o's, so every 32x32->64 product is one multiply-add with
+// carry in and out (a mad.lo.cc / madc.hi.cc pair on one aligned pair issues as one wide
+// multiply-add) and no separate additions fold it in.  Shifting the value down one limb
+// swaps the roles: o's pairs become the new even ones and e's the new odd ones, one column
+// lower, with e's second limb left over.  Every value below stays under 2^288 (9 limbs)
+// while a + c + p < 2^256, so o never carries out.
+// B200: a wide multiply-add with carry holds the multiply pipe for 4 cycles a warp, so a
+// product (128 of them and 8 low products) takes at least 528; measured 545 (68 G products/s
+// over the GPU) against 807 for wide products folded by add-with-carry chains (46 G/s) and
+// 651 for a radix-2^52 product on the FP64 pipe (57 G/s).  Warps of both kinds side by side
+// gain nothing over this one alone, nor does a Karatsuba a*b (112 multiply-adds, 577 cycles:
+// its additions cost what it saves).
+
+// e, o = a * b
+CSB_DEV void eo_mul(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a)[8], uint32_t b) {
+#pragma unroll
+  for (int k = 0; k < 8; k += 2) {
+    asm("mul.lo.u32 %0, %2, %3;\n\tmul.hi.u32 %1, %2, %3;" : "=&r"(e[k]), "=&r"(e[k + 1]) : "r"(a[k]), "r"(b));
+    asm("mul.lo.u32 %0, %2, %3;\n\tmul.hi.u32 %1, %2, %3;" : "=&r"(o[k]), "=&r"(o[k + 1]) : "r"(a[k + 1]), "r"(b));
+  }
+}
+// e, o += a * b
+CSB_DEV void eo_mad(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a)[8], uint32_t b) {
+  asm("{\n\t"
+      "mad.lo.cc.u32 %8, %17, %24, %8;\n\tmadc.hi.cc.u32 %9, %17, %24, %9;\n\t"
+      "madc.lo.cc.u32 %10, %19, %24, %10;\n\tmadc.hi.cc.u32 %11, %19, %24, %11;\n\t"
+      "madc.lo.cc.u32 %12, %21, %24, %12;\n\tmadc.hi.cc.u32 %13, %21, %24, %13;\n\t"
+      "madc.lo.cc.u32 %14, %23, %24, %14;\n\tmadc.hi.u32 %15, %23, %24, %15;\n\t"
+      "mad.lo.cc.u32 %0, %16, %24, %0;\n\tmadc.hi.cc.u32 %1, %16, %24, %1;\n\t"
+      "madc.lo.cc.u32 %2, %18, %24, %2;\n\tmadc.hi.cc.u32 %3, %18, %24, %3;\n\t"
+      "madc.lo.cc.u32 %4, %20, %24, %4;\n\tmadc.hi.cc.u32 %5, %20, %24, %5;\n\t"
+      "madc.lo.cc.u32 %6, %22, %24, %6;\n\tmadc.hi.cc.u32 %7, %22, %24, %7;\n\t"
+      "addc.u32 %15, %15, 0;\n\t}"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(o[0]),
+        "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b));
+}
+// (e, o) <- ((e, o) >> 32) + a * b, for e[0] = 0.  The left-over limb e[1] goes into the new
+// column 0 first; its carry (column 1) enters the odd chain, which starts there.
+CSB_DEV void eo_shift_mad(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a)[8], uint32_t b) {
+  uint32_t n0, n1, n2, n3, n4, n5, n6, n7;
+  asm("{\n\t"
+      "add.cc.u32 %0, %0, %16;\n\t"
+      "madc.lo.cc.u32 %8, %24, %31, %17;\n\tmadc.hi.cc.u32 %9, %24, %31, %18;\n\t"
+      "madc.lo.cc.u32 %10, %26, %31, %19;\n\tmadc.hi.cc.u32 %11, %26, %31, %20;\n\t"
+      "madc.lo.cc.u32 %12, %28, %31, %21;\n\tmadc.hi.cc.u32 %13, %28, %31, %22;\n\t"
+      "madc.lo.cc.u32 %14, %30, %31, 0;\n\tmadc.hi.u32 %15, %30, %31, 0;\n\t"
+      "mad.lo.cc.u32 %0, %23, %31, %0;\n\tmadc.hi.cc.u32 %1, %23, %31, %1;\n\t"
+      "madc.lo.cc.u32 %2, %25, %31, %2;\n\tmadc.hi.cc.u32 %3, %25, %31, %3;\n\t"
+      "madc.lo.cc.u32 %4, %27, %31, %4;\n\tmadc.hi.cc.u32 %5, %27, %31, %5;\n\t"
+      "madc.lo.cc.u32 %6, %29, %31, %6;\n\tmadc.hi.cc.u32 %7, %29, %31, %7;\n\t"
+      "addc.u32 %15, %15, 0;\n\t}"
+      : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7]), "=&r"(n0),
+        "=&r"(n1), "=&r"(n2), "=&r"(n3), "=&r"(n4), "=&r"(n5), "=&r"(n6), "=&r"(n7)
+      : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(a[0]), "r"(a[1]), "r"(a[2]),
+        "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b));
+#pragma unroll
+  for (int k = 0; k < 8; k++) e[k] = o[k];
+  o[0] = n0; o[1] = n1; o[2] = n2; o[3] = n3; o[4] = n4; o[5] = n5; o[6] = n6; o[7] = n7;
+}
+// r = (e + 2^32 o) >> 32, for e[0] = 0 and a value below 2^288
+CSB_DEV void eo_join(uint32_t (&r)[8], const uint32_t (&e)[8], const uint32_t (&o)[8]) {
+  ADD_CC(r[0], o[0], e[1]);  ADDC_CC(r[1], o[1], e[2]); ADDC_CC(r[2], o[2], e[3]); ADDC_CC(r[3], o[3], e[4]);
+  ADDC_CC(r[4], o[4], e[5]); ADDC_CC(r[5], o[5], e[6]); ADDC_CC(r[6], o[6], e[7]); ADDC(r[7], o[7], 0u);
 }
 
 template <class M>
@@ -261,54 +183,26 @@ struct Fp {
   CSB_DEV Fp neg() const { return zero() - *this; }
   CSB_DEV Fp dbl() const { return *this + *this; }
 
-  // CIOS Montgomery product with wide (IMAD.WIDE) row products.
-  static CSB_DEV Fp mul_wide(const Fp& a, const Fp& b) {
-    const uint32_t (&A)[8] = a.v;
+  // Montgomery product without the final conditional subtraction: below (a b + m p) / 2^256,
+  // that is (1 + 0.19 i j) p for a <= i p, b <= j p (p = 0.189 * 2^256).  Needs a + p below
+  // 2^256; b may be any 256-bit value.
+  static CSB_DEV Fp mul_raw(const Fp& a, const Fp& b) {
     const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
-    uint32_t t[9];
+    uint32_t e[8], o[8];
+    eo_mul(e, o, a.v, b.v[0]);
+    eo_mad(e, o, P, e[0] * M::NP0);
 #pragma unroll
-    for (int i = 0; i < 9; i++) t[i] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      row_mad_wide(t, A, b.v[i]);
-      const uint32_t m = t[0] * M::NP0;
-      row_mad_wide(t, P, m);
-#pragma unroll
-      for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-      t[8] = 0;
+    for (int i = 1; i < 8; i++) {
+      eo_shift_mad(e, o, a.v, b.v[i]);
+      eo_mad(e, o, P, e[0] * M::NP0);
     }
-    uint32_t r8[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) r8[i] = t[i];
-    reduce_once(r8);
     Fp r;
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = r8[i];
+    eo_join(r.v, e, o);
     return r;
   }
 
-  // ---- lazily reduced values in [0, 2p) (BN254: 4p < 2^256) --------------------------
-  // CIOS without the final conditional subtraction: for a, b < 2p the result is below
-  // (a b + m p) / 2^256 < (4p^2 + 2^256 p) / 2^256 < 2p.
-  static CSB_DEV Fp mul_wide_lazy(const Fp& a, const Fp& b) {
-    const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
-    uint32_t t[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) t[i] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      row_mad_wide(t, a.v, b.v[i]);
-      const uint32_t m = t[0] * M::NP0;
-      row_mad_wide(t, P, m);
-#pragma unroll
-      for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-      t[8] = 0;
-    }
-    Fp r;
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = t[i];
-    return r;
-  }
+  // ---- lazily reduced values in [0, 2p) (BN254: 4p < 2^256): products of two such values
+  // are below 2p without the final subtraction (1.76 p)
   static CSB_DEV Fp mul_lazy(const Fp& a, const Fp& b);
   // 2p, limb i
   static CSB_DEV uint32_t p2(int i) {
@@ -364,15 +258,15 @@ struct Fp {
 #if defined(CSB_MUL_NOINLINE)
     return fp_mul_call<M>(a, b);
 #else
-    return mul_wide(a, b);
+    return mul_raw(a, b).canon();
 #endif
   }
 
   CSB_DEV Fp sqr() const { return (*this) * (*this); }
 
-  // x -> x * R mod p (normal form to Montgomery); any 256-bit x < 2^256 is accepted
-  // because the CIOS bound only needs a*b < p * 2^256.
-  CSB_DEV Fp to_mont() const { return (*this) * r2(); }
+  // x -> x * R mod p (normal form to Montgomery); any 256-bit x is accepted: the product
+  // with r2 < p on the left is below 2p.
+  CSB_DEV Fp to_mont() const { return r2() * (*this); }
   CSB_DEV Fp from_mont() const {
     Fp o = zero();
     o.v[0] = 1;
@@ -459,27 +353,14 @@ struct Fp {
 using Fq = Fp<ModQ>;
 using Fr = Fp<ModR>;
 
-// ------------------------------------------------------------ Fq2 = Fq[u]/(u^2+1) ----
 template <class M>
 __device__ __noinline__ Fp<M> fp_mul_call(Fp<M> a, Fp<M> b) {
-#if CSB_DP52
-  Fp<M> r;
-  dp52::mont<M>(a.v, b.v, r.v);
-  return r.canon();
-#else
-  return Fp<M>::mul_wide(a, b);
-#endif
+  return Fp<M>::mul_raw(a, b).canon();
 }
 
 template <class M>
 __device__ __noinline__ Fp<M> fp_mul_lazy_call(Fp<M> a, Fp<M> b) {
-#if CSB_DP52
-  Fp<M> r;
-  dp52::mont<M>(a.v, b.v, r.v);
-  return r;
-#else
-  return Fp<M>::mul_wide_lazy(a, b);
-#endif
+  return Fp<M>::mul_raw(a, b);
 }
 
 template <class M>
@@ -487,10 +368,11 @@ CSB_DEV Fp<M> Fp<M>::mul_lazy(const Fp<M>& a, const Fp<M>& b) {
 #if defined(CSB_MUL_NOINLINE)
   return fp_mul_lazy_call<M>(a, b);
 #else
-  return mul_wide_lazy(a, b);
+  return mul_raw(a, b);
 #endif
 }
 
+// ------------------------------------------------------------ Fq2 = Fq[u]/(u^2+1) ----
 struct Fq2 {
   Fq c0, c1;
   static CSB_DEV Fq2 zero() { return {Fq::zero(), Fq::zero()}; }

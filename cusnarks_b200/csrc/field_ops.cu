@@ -8,6 +8,7 @@
 
 #include "../../include/cusnarks_b200.h"
 #include "curve.cuh"
+#include "dp52.cuh"
 #include "runtime.cuh"
 
 namespace {
