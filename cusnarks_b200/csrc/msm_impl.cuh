@@ -326,10 +326,14 @@ __global__ void k_task_emit(const uint32_t* __restrict__ offsets, uint32_t nb, u
   }
 }
 
-// Minimum resident blocks per SM asked of the compiler for the accumulation kernel (0 = no
-// register cap): G2 at 3 (168 registers: 12 warps per SM instead of 8, measured faster), G1
-// uncapped (caps spilled and measured slower).
-template <class F> struct AccMinBlocks { static constexpr int value = 0; };
+// Minimum resident blocks per SM asked of the compiler for the accumulation kernel: G1 at 4
+// (128 registers, what its inlined addition takes), G2 at 3 (168 registers: 12 warps per SM
+// instead of 8, measured faster).
+// The G1 accumulation is bound by its multiply-adds (the products of xyzz_madd_lazy): 2^20
+// fixed-base terms 2.18 ms, 5950 cycles per 32 additions and scheduler, against 2.44 ms with
+// the products called out of line and one reduction each; 3 and 5 blocks 2.18 and 2.15 ms (but
+// 2.79 against 2.71 ms over the GLV split's points), loading the next point ahead 2.18-2.25 ms.
+template <class F> struct AccMinBlocks { static constexpr int value = 4; };
 template <> struct AccMinBlocks<Fq2> { static constexpr int value = 3; };
 
 // The accumulation's mixed addition: over Fq with lazily reduced coordinates (no final
@@ -876,8 +880,10 @@ CSB_DEV uint32_t bucket_of_slot(const uint32_t* off, uint32_t nb, uint32_t s) {
   return lo;
 }
 
+// At least 3 blocks a SM asked for: over Fq2 the products take 198 registers uncapped, two
+// blocks (2^20 fixed-base G2 MSM 10.44 ms); at 168 registers, three blocks, 9.05 ms.
 template <class F, bool FIRST>
-__global__ void __launch_bounds__(128) k_affine_round(const uint32_t* __restrict__ in_off,
+__global__ void __launch_bounds__(128, 3) k_affine_round(const uint32_t* __restrict__ in_off,
                                                       const uint32_t* __restrict__ out_off, uint32_t nb,
                                                       const uint32_t* __restrict__ entries,
                                                       const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
