@@ -28,7 +28,8 @@ namespace {
 constexpr int kMaxLog = 27;
 
 // consts layout (Fr elements): 0 w_n, 1 w_n^-1, 2 n^-1 R (Montgomery), 3 n^-1 (normal),
-// 4 (n/2)^-1 R, 5 g, 6 g^-1, 7 (g^(n/2) - 1)^-1, 8 (n/2)^-1 (normal)
+// 4 (n/2)^-1 R, 5 g, 6 g^-1, 7 (g^(n/2) - 1)^-1, 8 (n/2)^-1 (normal), 9 n^-2 R
+constexpr size_t kConsts = 10;
 __global__ void k_domain_consts(uint32_t L, uint32_t* out) {
   if (threadIdx.x != 0) return;
   Fr w;
@@ -53,6 +54,7 @@ __global__ void k_domain_consts(uint32_t L, uint32_t* out) {
   for (uint32_t k = 1; k < L; k++) gm = gm.sqr();  // g^(n/2)
   st_fp<ModR>(out + 56, (gm - Fr::one()).inv());
   st_fp<ModR>(out + 64, hinv.from_mont());
+  st_fp<ModR>(out + 72, ninv.sqr());
 }
 
 // T[i] = s * g^-i as a normal-form value: a Montgomery product x*T[i] then yields
@@ -69,7 +71,7 @@ __global__ void k_scaled_normal(const uint32_t* __restrict__ pw, const uint32_t*
 // Twiddle and coset tables for transforms of 2^L points, resident in HBM per context.
 struct Domain {
   uint32_t L = 0;
-  uint32_t* consts = nullptr;  // 9 elements (see k_domain_consts)
+  uint32_t* consts = nullptr;  // see k_domain_consts
   uint32_t* Wf = nullptr;      // w^j, j < 2^(L-1)
   uint32_t* Wi = nullptr;      // w^-j
   uint32_t* G = nullptr;       // g^i, i < 2^(L-1)      (coset of the half-size domain)
@@ -109,7 +111,7 @@ cudaError_t domain_get(cs_ctx* ctx, uint32_t L, Domain** out) {
   d->L = L;
   const size_t half = (size_t)1 << (L - 1);
   cudaError_t e;
-  if ((e = cudaMalloc(&d->consts, 9 * 32)) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&d->consts, kConsts * 32)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&d->Wf, half * 32)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&d->Wi, half * 32)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&d->G, half * 32)) != cudaSuccess) return e;
@@ -140,69 +142,66 @@ const uint32_t* domain_consts(const Domain* d) { return d->consts; }
 // Reference semantics (src/cuda/ntt.cpp:778 interpol_and_mul_h): A, B evaluations on the
 // m-th roots (Montgomery) -> the 2m coefficients of A(x)B(x) in normal form.
 //   tabs: Wf2/Wi2 twiddles of the 2m-point domain, shift[i] (i < m) the odd-coset shift,
-//   minv_R = m^-1 (Montgomery), m2inv = (2m)^-1 (normal form).
+//   minv2_R = m^-2 (Montgomery), m2inv = (2m)^-1 (normal form).
+// A and B go through each transform side by side.  The even evaluations A o B and the odd ones
+// are formed as the last transform reads them, which also takes the two inverse transforms'
+// 1/m: three transforms and no elementwise pass.
 // Scratch: 4 m elements.  A and B are not modified.  batch instances: instance y's A, B,
 // out and scratch lie y * stride words after instance 0's (the tables are shared).
 cudaError_t hstep_reference_core(const uint32_t* A, const uint32_t* B, uint32_t L, const uint32_t* Wf2,
-                                 const uint32_t* Wi2, const uint32_t* shift, const uint32_t* minv_R,
+                                 const uint32_t* Wi2, const uint32_t* shift, const uint32_t* minv2_R,
                                  const uint32_t* m2inv, uint32_t* out, uint32_t* scratch, cudaStream_t st,
                                  uint32_t batch = 1, size_t stride = 0) {
   const size_t m = (size_t)1 << L;
-  uint32_t* E = scratch;
-  uint32_t* O = scratch + m * 8;
-  uint32_t* a = scratch + 2 * m * 8;
-  uint32_t* b = scratch + 3 * m * 8;
+  uint32_t* tmp = scratch;
+  uint32_t* ab = scratch + 2 * m * 8;  // a, then b
   cudaError_t e;
-  if ((e = fr_mul_batch(A, B, E, (uint32_t)m, batch, stride, st)) != cudaSuccess) return e;
   NttArgs t;
   t.batch = batch; t.stride = stride;
   t.log_n = L; t.log_tab = L + 1;
-  // a = shift * INTT_m(A), b likewise
-  t.in = A; t.out = a; t.W = Wi2; t.post_scalar = minv_R; t.post_tab = shift;
-  if ((e = ntt_run(t, st)) != cudaSuccess) return e;
-  t.in = B; t.out = b;
+  // a = m shift * INTT_m(A), b likewise
+  t.in[0] = A; t.in[1] = B; t.count = 2;
+  t.out = ab; t.out_step = m * 8;
+  t.W = Wi2; t.post_tab = shift; t.lazy_out = true;
   if ((e = ntt_run(t, st)) != cudaSuccess) return e;
   // odd-coset evaluations, in place
-  t.post_scalar = nullptr; t.post_tab = nullptr; t.W = Wf2;
-  t.in = a; t.out = a; t.tmp = O;
+  t.in[0] = ab; t.in[1] = ab + m * 8; t.tmp = tmp;
+  t.W = Wf2; t.post_tab = nullptr;
   if ((e = ntt_run(t, st)) != cudaSuccess) return e;
-  t.in = b; t.out = b; t.tmp = O;
-  if ((e = ntt_run(t, st)) != cudaSuccess) return e;
-  if ((e = fr_mul_batch(a, b, O, (uint32_t)m, batch, stride, st)) != cudaSuccess) return e;
   // 2m coefficients, normal form
   NttArgs u;
   u.batch = batch; u.stride = stride;
   u.log_n = L + 1; u.log_tab = L + 1;
-  u.in = E; u.in_odd = O; u.out = out; u.W = Wi2; u.post_scalar = m2inv;
+  u.load = NttLoad::kInterleaved;
+  u.in[0] = A; u.mul = B; u.odd = ab; u.odd_mul = ab + m * 8; u.scalar = minv2_R;
+  u.out = out; u.W = Wi2; u.post_scalar = m2inv;
   return ntt_run(u, st);
 }
 
 // Coset variant: H (m coefficients, normal form) of (A B - C) / (x^m - 1) evaluated on
 // g*<w>.  dom: the 2m-point domain (its G / Tinv cover m entries, w_m = Wf2 stride 2).
+// Scratch: 6 m elements.  The quotient is formed as the last transform reads it.
 cudaError_t hstep_coset_core(const uint32_t* A, const uint32_t* B, const uint32_t* C, uint32_t L,
                              const Domain* dom, uint32_t* out, uint32_t* scratch, cudaStream_t st) {
-  const size_t m = (size_t)1 << L;
-  uint32_t* a = scratch;
-  uint32_t* b = scratch + m * 8;
-  uint32_t* c = scratch + 2 * m * 8;
-  uint32_t* tmp = scratch + 3 * m * 8;
-  const uint32_t* src[3] = {A, B, C};
-  uint32_t* dst[3] = {a, b, c};
+  const size_t m = (size_t)1 << L, step = m * 8;
+  uint32_t* abc = scratch;
   cudaError_t e;
-  for (int k = 0; k < 3; k++) {
-    NttArgs t;
-    t.log_n = L; t.log_tab = L + 1; t.W = dom->Wi;
-    t.in = src[k]; t.out = dst[k]; t.post_scalar = dom->consts + 32; t.post_tab = dom->G;
-    if ((e = ntt_run(t, st)) != cudaSuccess) return e;
-    NttArgs f;
-    f.log_n = L; f.log_tab = L + 1; f.W = dom->Wf;
-    f.in = dst[k]; f.out = dst[k]; f.tmp = tmp;
-    if ((e = ntt_run(f, st)) != cudaSuccess) return e;
-  }
-  if ((e = fr_mul_sub_scale(a, b, c, dom->consts + 56, a, (uint32_t)m, st)) != cudaSuccess) return e;
+  NttArgs t;
+  t.log_n = L; t.log_tab = L + 1; t.W = dom->Wi;
+  t.in[0] = A; t.in[1] = B; t.in[2] = C; t.count = 3;
+  t.out = abc; t.out_step = step;
+  t.post_scalar = dom->consts + 32; t.post_tab = dom->G; t.lazy_out = true;
+  if ((e = ntt_run(t, st)) != cudaSuccess) return e;
+  for (int z = 0; z < 3; z++) t.in[z] = abc + z * step;
+  t.tmp = abc + 3 * step;
+  t.post_scalar = t.post_tab = nullptr;
+  t.W = dom->Wf; t.lazy_out = false;
+  if ((e = ntt_run(t, st)) != cudaSuccess) return e;
   NttArgs h;
   h.log_n = L; h.log_tab = L + 1; h.W = dom->Wi;
-  h.in = a; h.out = out; h.tmp = tmp; h.post_tab = dom->Tinv;
+  h.load = NttLoad::kQuotient;
+  h.in[0] = abc; h.mul = abc + step; h.sub = abc + 2 * step; h.scalar = dom->consts + 56;
+  h.out = out; h.post_tab = dom->Tinv;
   return ntt_run(h, st);
 }
 
@@ -269,13 +268,13 @@ int host_ntt(cs_ctx* ctx, uint32_t* A, const uint32_t* roots, uint32_t L, uint64
   uint32_t* dA = cv.take(bytes);
   uint32_t* dOut = cv.take(bytes);
   uint32_t* dW = cv.take(half * 32);
-  uint32_t* dC = cv.take(9 * 32);
+  uint32_t* dC = cv.take(kConsts * 32);
   if ((e = cudaMemcpyAsync(dA, src_host, bytes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
     return fail(ctx, e, "ntt H2D");
   if (half && (e = cudaMemcpyAsync(dW, W.data(), half * 32, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
     return fail(ctx, e, "ntt H2D roots");
   NttArgs t;
-  t.in = dA; t.out = dOut; t.log_n = L; t.log_tab = L; t.W = dW;
+  t.in[0] = dA; t.out = dOut; t.log_n = L; t.log_tab = L; t.W = dW;
   if (scale_fmat >= 0) {
     k_domain_consts<<<1, 32, 0, ctx->stream>>>(L, dC);
     note_launch();
@@ -382,8 +381,8 @@ uint32_t* ntt_interpolandmul_server_h(ntt_interpolandmul_t* args) {
   uint32_t* dS = cv.take(mb);
   uint32_t* dOut = cv.take(2 * mb);
   uint32_t* dScr = cv.take(4 * mb);
-  uint32_t* dCm = cv.take(9 * 32);   // m-point constants: [2] m^-1 R
-  uint32_t* dC2 = cv.take(9 * 32);   // 2m-point constants: [3] (2m)^-1 normal
+  uint32_t* dCm = cv.take(kConsts * 32);   // m-point constants: [9] m^-2 R
+  uint32_t* dC2 = cv.take(kConsts * 32);   // 2m-point constants: [3] (2m)^-1 normal
   std::vector<uint32_t>& res = interp_result();
   res.assign(2 * m * 8, 0u);
   bool ok = (e = cudaMemcpyAsync(dA, args->A, mb, cudaMemcpyHostToDevice, ctx->stream)) == cudaSuccess &&
@@ -396,7 +395,7 @@ uint32_t* ntt_interpolandmul_server_h(ntt_interpolandmul_t* args) {
     k_domain_consts<<<1, 32, 0, ctx->stream>>>(L + 1, dC2);
     note_launch(2);
     cudaEventRecord(ctx->ev_start, ctx->stream);
-    e = hstep_reference_core(dA, dB, L, dWf, dWi, dS, dCm + 16, dC2 + 24, dOut, dScr, ctx->stream);
+    e = hstep_reference_core(dA, dB, L, dWf, dWi, dS, dCm + 72, dC2 + 24, dOut, dScr, ctx->stream);
     cudaEventRecord(ctx->ev_stop, ctx->stream);
     ok = e == cudaSuccess &&
          (e = cudaMemcpyAsync(res.data(), dOut, 2 * mb, cudaMemcpyDeviceToHost, ctx->stream)) == cudaSuccess &&
@@ -472,7 +471,7 @@ int cs_ntt_device(cs_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint32_t l
     if ((e = ctx->work.reserve(bytes, ctx->stream)) != cudaSuccess) return fail(ctx, e, "ntt scratch");
   }
   NttArgs t;
-  t.in = d_in; t.out = d_out; t.tmp = static_cast<uint32_t*>(ctx->work.ptr);
+  t.in[0] = d_in; t.out = d_out; t.tmp = static_cast<uint32_t*>(ctx->work.ptr);
   t.log_n = log_n; t.log_tab = log_n;
   t.W = direction >= 0 ? dom->Wf : dom->Wi;
   if (direction < 0) t.post_scalar = dom->consts + (fmat ? 16 : 24);
@@ -495,11 +494,11 @@ int cs_hstep_device(cs_ctx* ctx, int variant, const uint32_t* d_A, const uint32_
   if (e == cudaSuccess) e = domain_get(ctx, log_m, &dom1);
   if (e != cudaSuccess) return fail(ctx, e, "hstep domain");
   const size_t mb = (size_t)32 << log_m;
-  if ((e = ctx->work.reserve(4 * mb, ctx->stream)) != cudaSuccess) return fail(ctx, e, "hstep scratch");
+  if ((e = ctx->work.reserve((variant == CS_HSTEP_COSET ? 6 : 4) * mb, ctx->stream)) != cudaSuccess) return fail(ctx, e, "hstep scratch");
   uint32_t* scr = static_cast<uint32_t*>(ctx->work.ptr);
   cudaEventRecord(ctx->ev_start, ctx->stream);
   if (variant == CS_HSTEP_REFERENCE)
-    e = hstep_reference_core(d_A, d_B, log_m, dom2->Wf, dom2->Wi, dom2->Wf, dom1->consts + 16,
+    e = hstep_reference_core(d_A, d_B, log_m, dom2->Wf, dom2->Wi, dom2->Wf, dom1->consts + 72,
                              dom2->consts + 24, d_out, scr, ctx->stream);
   else
     e = hstep_coset_core(d_A, d_B, d_C, log_m, dom2, d_out, scr, ctx->stream);

@@ -1,4 +1,6 @@
 // ntt.cu -- radix-2 NTT passes in shared memory and Fr elementwise helpers (ntt.cuh).
+#include <algorithm>
+
 #include "ntt.cuh"
 #include "curve.cuh"
 #include "runtime.cuh"
@@ -9,70 +11,185 @@ namespace {
 
 constexpr int kMaxStages = 11;  // 2^11 elements x 32 B = 64 KB of shared memory per block
 constexpr int kThreads = 256;
-
-CSB_DEV void lds_fr(Fr& x, const uint4* s, uint32_t i) {
-  const uint4 a = s[2 * i], b = s[2 * i + 1];
-  x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
-  x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
-}
-CSB_DEV void sts_fr(uint4* s, uint32_t i, const Fr& x) {
-  s[2 * i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-  s[2 * i + 1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
+// One thread per butterfly (k_ntt_pass2) up to this many warps a scheduler, beyond it a thread
+// per four elements (us, at 1 / 4 / 8: H step of 2^15 97 / 79 / 79, of 2^16 123.6 / 116.5 / 116.4,
+// of 2^17 196.0 / 196.1 / 199.1; NTT 2^18 66.8 / 66.8 / 70.4).
+constexpr uint64_t kLatencyWarps = 4;
 
 // One pass: stages s0 .. s0+S-1 of a radix-2 DIT transform of 2^L points.  Block q owns
 // the 2^S elements base + (i << s0), base = ((q >> s0) << (s0 + S)) + (q & (2^s0 - 1)).
-// blockIdx.y: the instance of a batch, its arrays `stride` words after the previous one's.
-__global__ void __launch_bounds__(kThreads) k_ntt_pass(
-    const uint32_t* __restrict__ in, const uint32_t* __restrict__ in_odd, uint32_t* out,
-    uint32_t L, uint32_t s0, uint32_t S, int bitrev, const uint32_t* __restrict__ W,
-    uint32_t wshift, const uint32_t* __restrict__ post_tab, const uint32_t* __restrict__ post_scalar,
-    size_t stride) {
-  extern __shared__ uint4 sm[];
-  const size_t inst = (size_t)blockIdx.y * stride;
-  in += inst;
-  if (in_odd) in_odd += inst;
-  out += inst;
-  const uint32_t q = blockIdx.x;
-  const uint32_t rmask = (1u << s0) - 1u;
-  const uint64_t base = ((uint64_t)(q >> s0) << (s0 + S)) + (q & rmask);
-  const uint32_t cnt = 1u << S;
-  for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const uint64_t g = base + ((uint64_t)i << s0);
-    uint64_t src = g;
-    if (bitrev) src = __brev((uint32_t)g) >> (32 - L);
-    const uint32_t* p = in_odd ? ((src & 1) ? in_odd : in) + (src >> 1) * 8 : in + src * 8;
-    Fr x = ld_fp<ModR>(p);
-    sts_fr(sm, i, x);
+// blockIdx.y: the instance of a batch, its arrays `stride` words after the previous one's;
+// blockIdx.z: the transform (NttArgs::count).
+struct Pass {
+  const uint32_t* in[3];
+  uint32_t* out;
+  const uint32_t *mul, *odd, *odd_mul, *sub, *scalar;
+  const uint32_t *W, *post_tab, *post_scalar;
+  size_t stride, in_step, out_step;  // in_step: offset of in[0] per transform where in[1] is null
+  uint32_t L, s0, S, wshift;
+  int bitrev, load, canon;
+};
+
+// Element g of the pass's input, below 4r.
+CSB_DEV Fr pass_load(const Pass& a, const uint32_t* in, size_t inst, uint32_t g) {
+  if (!a.bitrev) return ld_fp<ModR>(in + (size_t)g * 8);
+  const uint32_t i = __brev(g) >> (32 - a.L);
+  if (a.load == (int)NttLoad::kPlain) return ld_fp<ModR>(in + (size_t)i * 8);
+  if (a.load == (int)NttLoad::kInterleaved) {
+    const size_t o = inst + (size_t)(i >> 1) * 8;
+    if ((i & 1) == 0) return Fr::mul_raw(ld_fp<ModR>(in + (size_t)(i >> 1) * 8), ld_fp<ModR>(a.mul + o));
+    return Fr::mul_raw(Fr::mul_raw(ld_fp<ModR>(a.odd + o), ld_fp<ModR>(a.odd_mul + o)), ld_fp<ModR>(a.scalar));
   }
-  __syncthreads();
-  const uint32_t r = q & rmask;
-  for (uint32_t t = 0; t < S; t++) {
-    const uint32_t s = s0 + t;
-    const uint32_t tmask = (1u << t) - 1u;
-    const uint32_t tw_shift = L - s - 1 + wshift;
-    for (uint32_t b = threadIdx.x; b < cnt / 2; b += blockDim.x) {
-      const uint32_t lo = ((b >> t) << (t + 1)) | (b & tmask);
-      const uint32_t hi = lo + (1u << t);
-      const uint64_t k = (uint64_t)r + ((uint64_t)(lo & tmask) << s0);
-      Fr x, y;
-      lds_fr(x, sm, lo);
-      lds_fr(y, sm, hi);
-      if (k != 0) y = y * ld_fp<ModR>(W + (k << tw_shift) * 8);
-      sts_fr(sm, lo, x + y);
-      sts_fr(sm, hi, x - y);
+  const size_t o = inst + (size_t)i * 8;
+  const Fr ab = Fr::mul_raw(ld_fp<ModR>(in + (size_t)i * 8), ld_fp<ModR>(a.mul + o));  // < 1.2r
+  return Fr::mul_raw(Fr::sub_lazy(ab, ld_fp<ModR>(a.sub + o)), ld_fp<ModR>(a.scalar));
+}
+// Element g of the pass's output from x < 4r.
+CSB_DEV void pass_store(const Pass& a, uint32_t* out, uint32_t g, Fr x) {
+  if (a.post_scalar) x = Fr::mul_raw(x, ld_fp<ModR>(a.post_scalar));
+  if (a.post_tab) x = Fr::mul_raw(x, ld_fp<ModR>(a.post_tab + (size_t)g * 8));
+  if (a.canon) x = Fr::reduce_2p(x).canon();
+  st_fp<ModR>(out + (size_t)g * 8, x);
+}
+// Butterfly on values below 4r (4r < 2^256): x, y -> x + t, x - t with t = w y < 2r, both
+// below 4r again: one conditional subtraction of 2r instead of three reductions to [0, r).
+CSB_DEV void butterfly(Fr& x, Fr& y, const Fr& t) {
+  const Fr u = Fr::reduce_2p(x);
+  x = Fr::add_raw(u, t);
+  y = Fr::add_raw(u, Fr::neg_lazy(t));
+}
+
+// Elements as two arrays of 16-byte halves: lanes read consecutive 16-byte words, where
+// whole 32-byte elements would meet in half the banks.
+struct Tile {
+  uint4 *lo, *hi;
+  CSB_DEV Fr get(uint32_t i) const {
+    const uint4 a = lo[i], b = hi[i];
+    return Fr{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+  }
+  CSB_DEV void put(uint32_t i, const Fr& x) const {
+    lo[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
+    hi[i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+  }
+};
+
+struct Block {
+  const uint32_t* in;
+  uint32_t* out;
+  size_t inst;
+  uint32_t r, base;
+};
+CSB_DEV Block pass_block(const Pass& a) {
+  Block b;
+  b.inst = (size_t)blockIdx.y * a.stride;
+  const uint32_t z = blockIdx.z;
+  b.in = (a.in[1] ? a.in[z] : a.in[0] + z * a.in_step) + b.inst;
+  b.out = a.out + b.inst + z * a.out_step;
+  uint32_t q = blockIdx.x;
+  // the first pass's gather leaves a block's neighbours in memory to blocks 2^(L-S-1) and
+  // 2^(L-S-2) further on: four consecutive blocks share their 128-byte lines this way
+  if (a.bitrev && a.L - a.S >= 2) q = (q >> 2) | ((q & 3u) << (a.L - a.S - 2));
+  const uint32_t rmask = (1u << a.s0) - 1u;
+  b.r = q & rmask;
+  b.base = ((q >> a.s0) << (a.s0 + a.S)) + b.r;
+  return b;
+}
+
+// Throughput form (2^22 points 0.89 ms, 1.05 ms with one stage a barrier and values reduced below r
+// after each; bound by the products, 0.68 ms at the GPU's rate): a thread takes four elements through two stages at a time, so a pass
+// crosses shared memory and the barrier (S - 1) / 2 times; the first stages read from and
+// the last write to global memory directly.  An odd S starts with one single stage.  Three
+// blocks a SM (84 registers) gain 2 % from 2^20 on and lose 5 % at 2^17 to 2^19.
+__global__ void __launch_bounds__(kThreads, 2) k_ntt_pass4(const Pass a) {
+  extern __shared__ uint4 sm[];
+  const uint32_t cnt = 1u << a.S, s0 = a.s0;
+  const Tile tile{sm, sm + cnt};
+  const Block b = pass_block(a);
+  uint32_t t = 0;
+  if (a.S & 1) {
+    const Fr w = ld_fp<ModR>(a.W + ((size_t)b.r << (a.L - s0 - 1 + a.wshift)) * 8);
+#pragma unroll 1
+    for (uint32_t j = threadIdx.x; j < cnt / 2; j += blockDim.x) {
+      Fr x = pass_load(a, b.in, b.inst, b.base + ((2 * j) << s0));
+      Fr y = pass_load(a, b.in, b.inst, b.base + ((2 * j + 1) << s0));
+      butterfly(x, y, s0 == 0 ? Fr::reduce_2p(y) : Fr::mul_raw(y, w));
+      tile.put(2 * j, x);
+      tile.put(2 * j + 1, y);
+    }
+    t = 1;
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (; t < a.S; t += 2) {
+    const bool first = t == 0, last = t + 2 == a.S;
+    const uint32_t sh = a.L - (s0 + t) - 2 + a.wshift;  // of the second stage's twiddles
+#pragma unroll 1
+    for (uint32_t j = threadIdx.x; j < cnt / 4; j += blockDim.x) {
+      const uint32_t low = j & ((1u << t) - 1u);
+      const uint32_t i0 = ((j >> t) << (t + 2)) | low;
+      const uint32_t k = b.r + (low << s0);
+      Fr x[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint32_t i = i0 + ((uint32_t)q << t);
+        x[q] = first ? pass_load(a, b.in, b.inst, b.base + (i << s0)) : tile.get(i);
+      }
+      if (first && s0 == 0) {  // twiddles 1, 1 and 1, w^(n/4)
+        butterfly(x[0], x[1], Fr::reduce_2p(x[1]));
+        butterfly(x[2], x[3], Fr::reduce_2p(x[3]));
+        butterfly(x[0], x[2], Fr::reduce_2p(x[2]));
+      } else {
+        const Fr w1 = ld_fp<ModR>(a.W + ((size_t)k << (sh + 1)) * 8);
+        butterfly(x[0], x[1], Fr::mul_raw(x[1], w1));
+        butterfly(x[2], x[3], Fr::mul_raw(x[3], w1));
+        butterfly(x[0], x[2], Fr::mul_raw(x[2], ld_fp<ModR>(a.W + ((size_t)k << sh) * 8)));
+      }
+      butterfly(x[1], x[3], Fr::mul_raw(x[3], ld_fp<ModR>(a.W + ((size_t)(k + (1u << (s0 + t))) << sh) * 8)));
+      if (first && last) __syncthreads();  // one round: every element read before any is written
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const uint32_t i = i0 + ((uint32_t)q << t);
+        if (last) pass_store(a, b.out, b.base + (i << s0), x[q]);
+        else tile.put(i, x[q]);
+      }
     }
     __syncthreads();
   }
-  Fr sc;
-  if (post_scalar) sc = ld_fp<ModR>(post_scalar);
-  for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const uint64_t g = base + ((uint64_t)i << s0);
-    Fr x;
-    lds_fr(x, sm, i);
-    if (post_scalar) x = x * sc;
-    if (post_tab) x = x * ld_fp<ModR>(post_tab + g * 8);
-    st_fp<ModR>(out + g * 8, x);
+}
+
+// Latency form, for transforms that leave schedulers idle: a thread per butterfly, one stage
+// at a time (a stage is one product deep), the next stage's twiddle loaded ahead.
+__global__ void __launch_bounds__(1024) k_ntt_pass2(const Pass a) {
+  extern __shared__ uint4 sm[];
+  const uint32_t cnt = 1u << a.S, s0 = a.s0, j = threadIdx.x;
+  const Tile tile{sm, sm + cnt};
+  const Block b = pass_block(a);
+  auto twiddle = [&](uint32_t t) {
+    const uint32_t k = b.r + ((j & ((1u << t) - 1u)) << s0);
+    return ld_fp<ModR>(a.W + ((size_t)k << (a.L - (s0 + t) - 1 + a.wshift)) * 8);
+  };
+  Fr w = twiddle(0);
+  Fr x = pass_load(a, b.in, b.inst, b.base + ((2 * j) << s0));
+  Fr y = pass_load(a, b.in, b.inst, b.base + ((2 * j + 1) << s0));
+#pragma unroll 1
+  for (uint32_t t = 0;; t++) {
+    const uint32_t i = ((j >> t) << (t + 1)) | (j & ((1u << t) - 1u));
+    const Fr wn = t + 1 < a.S ? twiddle(t + 1) : w;
+    if (t) {
+      x = tile.get(i);
+      y = tile.get(i + (1u << t));
+    }
+    butterfly(x, y, Fr::mul_raw(y, w));
+    w = wn;
+    if (t + 1 == a.S) {
+      if (t == 0) __syncthreads();  // one stage: every element read before any is written
+      pass_store(a, b.out, b.base + (i << s0), x);
+      pass_store(a, b.out, b.base + ((i + (1u << t)) << s0), y);
+      return;
+    }
+    tile.put(i, x);
+    tile.put(i + (1u << t), y);
+    __syncthreads();
   }
 }
 
@@ -108,29 +225,16 @@ __global__ void k_gather_roots(uint32_t* __restrict__ out, const uint32_t* __res
   d[1] = s[1];
 }
 
-__global__ void k_fr_mul(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                         uint32_t* __restrict__ out, uint32_t n, size_t stride) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const size_t o = (size_t)blockIdx.y * stride + (size_t)i * 8;
-  st_fp<ModR>(out + o, ld_fp<ModR>(a + o) * ld_fp<ModR>(b + o));
-}
-
-__global__ void k_fr_mul_sub_scale(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                                   const uint32_t* __restrict__ c, const uint32_t* __restrict__ s,
-                                   uint32_t* __restrict__ out, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const Fr v = ld_fp<ModR>(a + (size_t)i * 8) * ld_fp<ModR>(b + (size_t)i * 8) - ld_fp<ModR>(c + (size_t)i * 8);
-  st_fp<ModR>(out + (size_t)i * 8, v * ld_fp<ModR>(s));
-}
-
+// Stages per pass.  At least two passes from 2^9 points on: one block would run alone on its
+// SM otherwise (2^11 points 50 us in one pass, 17 in two).  Two passes of equal odd size shift
+// one stage, an even number of stages needs no single one (k_ntt_pass4).
 void plan_passes(uint32_t L, uint32_t* sizes, int* np) {
-  const int n = (int)((L + kMaxStages - 1) / kMaxStages);
+  const int n = std::max((int)((L + kMaxStages - 1) / kMaxStages), L >= 9 ? 2 : 1);
   int k = 0;
   uint32_t left = L;
   for (int p = 0; p < n; p++) {
-    const uint32_t sz = (left + (n - p) - 1) / (n - p);  // even split, larger first
+    uint32_t sz = (left + (n - p) - 1) / (n - p);  // even split, larger first
+    if (n == 2 && p == 0 && sz * 2 == L && (sz & 1) && sz < (uint32_t)kMaxStages) sz++;
     sizes[k++] = sz;
     left -= sz;
   }
@@ -141,34 +245,57 @@ void plan_passes(uint32_t L, uint32_t* sizes, int* np) {
 
 cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
   const uint32_t L = a.log_n;
-  if (L == 0 || L > 28 || a.log_tab < L || !a.W || !a.in || !a.out || a.batch == 0 || a.batch > 65535)
+  if (L == 0 || L > 28 || a.log_tab < L || !a.W || !a.in[0] || !a.out || a.batch == 0 || a.batch > 65535 ||
+      a.count == 0 || a.count > 3)
     return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_ntt_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << kMaxStages) * 32);
-    attr_set = true;
-  }
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   uint32_t sizes[8];
   int np = 0;
   plan_passes(L, sizes, &np);
-  const bool alias = (a.in == a.out) || (a.in_odd == a.out);
   uint32_t* work = a.out;
-  if (alias && np > 1) {
-    if (!a.tmp) return cudaErrorInvalidValue;
-    work = a.tmp;
+  if (np > 1) {
+    bool alias = false;
+    for (uint32_t z = 0; z < a.count; z++) alias |= a.in[z] == a.out + z * a.out_step;
+    if (alias) {
+      if (!a.tmp) return cudaErrorInvalidValue;
+      work = a.tmp;
+    }
   }
+  // one thread per butterfly while that leaves at most kLatencyWarps warps a scheduler
+  const bool latency = ((uint64_t)a.count * a.batch << (L - 1)) <= (uint64_t)sms * 4 * 32 * kLatencyWarps;
   uint32_t s0 = 0;
   for (int p = 0; p < np; p++) {
     const uint32_t S = sizes[p];
     const bool first = (p == 0), last = (p == np - 1);
-    const uint32_t* src = first ? a.in : work;
-    const uint32_t* src_odd = first ? a.in_odd : nullptr;
-    uint32_t* dst = last ? a.out : work;
-    const unsigned blocks = 1u << (L - S);
-    const unsigned threads = (1u << (S - 1)) < (unsigned)kThreads ? (1u << (S - 1)) : (unsigned)kThreads;
-    k_ntt_pass<<<dim3(blocks, a.batch), threads > 0 ? threads : 1, (1u << S) * 32, st>>>(
-        src, src_odd, dst, L, s0, S, first ? 1 : 0, a.W, a.log_tab - L,
-        last ? a.post_tab : nullptr, last ? a.post_scalar : nullptr, a.stride);
+    Pass q{};
+    for (int z = 0; z < 3; z++) q.in[z] = first ? (z < (int)a.count ? a.in[z] : nullptr) : nullptr;
+    if (!first) q.in[0] = work;
+    q.in_step = a.out_step;
+    q.out = last ? a.out : work;
+    q.out_step = a.out_step;
+    q.stride = a.stride;
+    q.mul = a.mul; q.odd = a.odd; q.odd_mul = a.odd_mul; q.sub = a.sub; q.scalar = a.scalar;
+    q.W = a.W;
+    q.post_tab = last ? a.post_tab : nullptr;
+    q.post_scalar = last ? a.post_scalar : nullptr;
+    q.L = L; q.s0 = s0; q.S = S; q.wshift = a.log_tab - L;
+    q.bitrev = first ? 1 : 0;
+    q.load = (int)a.load;
+    q.canon = last && !a.lazy_out;
+    const dim3 grid(1u << (L - S), a.batch, a.count);
+    if ((32u << S) > 48u * 1024) {  // above the default limit of a block's shared memory
+      const cudaError_t e = cudaFuncSetAttribute(latency ? (const void*)k_ntt_pass2 : (const void*)k_ntt_pass4,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 32 << S);
+      if (e != cudaSuccess) return e;
+    }
+    if (latency || S == 1) {
+      k_ntt_pass2<<<grid, 1u << (S - 1), (1u << S) * 32, st>>>(q);
+    } else {
+      const unsigned threads = (1u << (S - 2)) < (unsigned)kThreads ? (1u << (S - 2)) : (unsigned)kThreads;
+      k_ntt_pass4<<<grid, threads, (1u << S) * 32, st>>>(q);
+    }
     note_launch();
     s0 += S;
   }
@@ -188,31 +315,6 @@ cudaError_t ntt_gather_roots(uint32_t* d_out, const uint32_t* d_table, uint64_t 
                              int dir, uint32_t count, cudaStream_t st) {
   if (count == 0) return cudaSuccess;
   k_gather_roots<<<(count + 255) / 256, 256, 0, st>>>(d_out, d_table, stride, n, dir, count);
-  note_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t fr_mul(const uint32_t* a, const uint32_t* b, uint32_t* out, uint32_t n, cudaStream_t st) {
-  return fr_mul_batch(a, b, out, n, 1, 0, st);
-}
-
-cudaError_t fr_mul_batch(const uint32_t* a, const uint32_t* b, uint32_t* out, uint32_t n, uint32_t batch,
-                         size_t stride, cudaStream_t st) {
-  if (n == 0 || batch == 0) return cudaSuccess;
-  if (batch > 65535) return cudaErrorInvalidValue;
-  k_fr_mul<<<dim3((n + 255) / 256, batch), 256, 0, st>>>(a, b, out, n, stride);
-  note_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t fr_mul_tab(const uint32_t* a, const uint32_t* tab, uint32_t* out, uint32_t n, cudaStream_t st) {
-  return fr_mul(a, tab, out, n, st);
-}
-
-cudaError_t fr_mul_sub_scale(const uint32_t* a, const uint32_t* b, const uint32_t* c, const uint32_t* s,
-                             uint32_t* out, uint32_t n, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  k_fr_mul_sub_scale<<<(n + 255) / 256, 256, 0, st>>>(a, b, c, s, out, n);
   note_launch();
   return cudaGetLastError();
 }

@@ -38,7 +38,7 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
 cudaError_t batch_enqueue(cs_msm_batch* b, cudaStream_t st);
 cudaError_t domain_get(cs_ctx* ctx, uint32_t L, Domain** out);
 cudaError_t hstep_reference_core(const uint32_t* A, const uint32_t* B, uint32_t L, const uint32_t* Wf2,
-                                 const uint32_t* Wi2, const uint32_t* shift, const uint32_t* minv_R,
+                                 const uint32_t* Wi2, const uint32_t* shift, const uint32_t* minv2_R,
                                  const uint32_t* m2inv, uint32_t* out, uint32_t* scratch, cudaStream_t st,
                                  uint32_t batch = 1, size_t stride = 0);
 // accessors into the opaque Domain (hstep.cu)
@@ -318,7 +318,7 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
   ok = (e = qap_eval(pk->rows_a, d_w, pA, 0, sh)) == cudaSuccess &&
        (e = qap_eval(pk->rows_b, d_w, pB, 0, sh)) == cudaSuccess &&
        (e = hstep_reference_core(pA, pB, pk->log_m, domain_wf(dom2), domain_wi(dom2), domain_wf(dom2),
-                                 domain_consts(dom1) + 16, domain_consts(dom2) + 24, M, hscr, sh)) == cudaSuccess &&
+                                 domain_consts(dom1) + 72, domain_consts(dom2) + 24, M, hscr, sh)) == cudaSuccess &&
        (e = cudaEventRecord(ctx->aux_ev[6], sh)) == cudaSuccess &&  // H step done (stage times)
        // polH = M[m .. 2m-2]; M[2m-1] (always zero) becomes the -rs term for delta_1
        (e = cudaMemcpyAsync(M + (size_t)(2 * m - 1) * 8, rs + 16, 32, cudaMemcpyDeviceToDevice, sh)) == cudaSuccess &&
@@ -527,7 +527,7 @@ cudaError_t prove_batch_body(cs_ctx* ctx, cs_pk* pk, ProveBatch& B, Domain* dom1
         (e = qap_eval(pk->rows_a, B.at(0, B.o_wA), B.at(0, B.o_pA), 0, sh, K, stride)) == cudaSuccess &&
         (e = qap_eval(pk->rows_b, B.at(0, B.o_wA), B.at(0, B.o_pB), 0, sh, K, stride)) == cudaSuccess &&
         (e = hstep_reference_core(B.at(0, B.o_pA), B.at(0, B.o_pB), pk->log_m, domain_wf(dom2), domain_wi(dom2),
-                                  domain_wf(dom2), domain_consts(dom1) + 16, domain_consts(dom2) + 24,
+                                  domain_wf(dom2), domain_consts(dom1) + 72, domain_consts(dom2) + 24,
                                   B.at(0, B.o_M), B.at(0, B.o_hscr), sh, K, stride)) == cudaSuccess;
     if (!ok) { *where = "prove batch QAP/H"; return e; }
     k_batch_rs<<<K, 8, 0, sh>>>(base, B.per, B.o_rs, B.o_M, m);
