@@ -95,6 +95,7 @@ CSB_DEV XYZZ<F> xyzz_madd(const XYZZ<F>& p, const Affine<F>& q) {
   }
 }
 
+// out of line: the rare equal points of a bucket do not weigh on the addition's registers
 template <class F>
 __device__ __noinline__ XYZZ<F> xyzz_mdbl_cold(const Affine<F> p) { return xyzz_mdbl(p); }
 
@@ -156,137 +157,6 @@ CSB_DEV XYZZ<F> xyzz_add(const XYZZ<F>& p, const XYZZ<F>& q) {
 // code size and compile time in check, notably over Fq2.
 template <class F>
 __device__ __noinline__ XYZZ<F> xyzz_add_cold(const XYZZ<F> p, const XYZZ<F> q) { return xyzz_add(p, q); }
-template <class F>
-__device__ __noinline__ XYZZ<F> xyzz_dbl_cold(const XYZZ<F> p) { return xyzz_dbl(p); }
-
-// ------------------------------------------------ quad-parallel point operations -----
-// For chains that a point runs through alone (window Horner, scalar multiplication, the
-// buckets of a small MSM): the lanes of an aligned group hold the same point and each
-// computes part of the independent products of a dependency level, so a doubling costs 3
-// product latencies instead of 9, an addition 4 instead of 14 and a mixed addition 4
-// instead of 10.  A group is 4 lanes over Fq (a "quad": one product each) and 16 lanes over
-// Fq2 (twelve of them one Fq product each of the level's four Karatsuba products).  The
-// shuffles use the full warp mask, so every lane of the warp must call these together (the
-// warp's groups may hold different points: the special cases -- infinity, equal or opposite
-// points -- are selected after the general formula, never branched around it); every lane of
-// a group returns the same result.  The names keep "quad" for the group.
-template <class F> struct GroupLanes { static constexpr int value = 4; };
-template <> struct GroupLanes<Fq2> { static constexpr int value = 16; };
-
-template <int G, class T>
-CSB_DEV T grp_bcast(const T& v, int src) {
-  constexpr int TW = sizeof(T) / 4;
-  T o;
-  uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-  const uint32_t* vw = reinterpret_cast<const uint32_t*>(&v);
-#pragma unroll
-  for (int w = 0; w < TW; w++) ow[w] = __shfl_sync(0xffffffffu, vw[w], src, G);
-  return o;
-}
-template <class F>
-CSB_DEV F quad_bcast(const F& v, int src) { return grp_bcast<4>(v, src); }
-
-template <class F>
-CSB_DEV F pick4(int k, const F& v0, const F& v1, const F& v2, const F& v3) {
-  return k == 0 ? v0 : k == 1 ? v1 : k == 2 ? v2 : v3;
-}
-
-template <class F>
-CSB_DEV XYZZ<F> xyzz_select(bool c, const XYZZ<F>& a, const XYZZ<F>& b) { return c ? a : b; }
-
-// quad lane k computes a_k * b_k; every lane gets the four products
-template <class F>
-CSB_DEV void quad_mul4(const F& a0, const F& b0, const F& a1, const F& b1, const F& a2, const F& b2,
-                       const F& a3, const F& b3, F& r0, F& r1, F& r2, F& r3) {
-  const int k = threadIdx.x & 3;
-  const F r = pick4(k, a0, a1, a2, a3) * pick4(k, b0, b1, b2, b3);
-  r0 = quad_bcast(r, 0);
-  r1 = quad_bcast(r, 1);
-  r2 = quad_bcast(r, 2);
-  r3 = quad_bcast(r, 3);
-}
-// Over Fq2, in groups of 16 lanes: lane l < 12 computes part l mod 3 of Karatsuba product
-// l / 3 (a0 b0, a1 b1 or (a0 + a1)(b0 + b1), the Fq products Fq2's operator* forms), every lane
-// gathers the twelve and forms the four products as operator* does: the same bits, one Fq
-// product latency per level instead of three.
-template <>
-CSB_DEV void quad_mul4<Fq2>(const Fq2& a0, const Fq2& b0, const Fq2& a1, const Fq2& b1, const Fq2& a2,
-                            const Fq2& b2, const Fq2& a3, const Fq2& b3, Fq2& r0, Fq2& r1, Fq2& r2, Fq2& r3) {
-  const int l = threadIdx.x & 15;
-  const int j = l < 12 ? l / 3 : 0, part = l < 12 ? l - 3 * j : 0;
-  const Fq2 a = pick4(j, a0, a1, a2, a3), b = pick4(j, b0, b1, b2, b3);
-  const Fq x = part == 0 ? a.c0 : (part == 1 ? a.c1 : a.c0 + a.c1);
-  const Fq y = part == 0 ? b.c0 : (part == 1 ? b.c1 : b.c0 + b.c1);
-  const Fq p = x * y;
-  Fq2 r[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const Fq v0 = grp_bcast<16>(p, 3 * k), v1 = grp_bcast<16>(p, 3 * k + 1), s = grp_bcast<16>(p, 3 * k + 2);
-    r[k] = Fq2{v0 - v1, s - v0 - v1};
-  }
-  r0 = r[0];
-  r1 = r[1];
-  r2 = r[2];
-  r3 = r[3];
-}
-
-// dbl-2008-s-1, three levels of products
-template <class F>
-CSB_DEV XYZZ<F> xyzz_dbl_quad(const XYZZ<F>& p) {
-  const F U = p.Y.dbl();
-  F V, X2, W, S, MM, ZZ3, T1, T2, ZZZ3, unused;
-  quad_mul4(U, U, p.X, p.X, U, U, p.X, p.X, V, X2, unused, unused);
-  const F M = X2.dbl() + X2;
-  quad_mul4(U, V, p.X, V, M, M, V, p.ZZ, W, S, MM, ZZ3);
-  XYZZ<F> r;
-  r.X = MM - S.dbl();
-  quad_mul4(M, S - r.X, W, p.Y, W, p.ZZZ, W, p.ZZZ, T1, T2, ZZZ3, unused);
-  r.Y = T1 - T2;
-  r.ZZ = ZZ3;
-  r.ZZZ = ZZZ3;
-  return xyzz_select(p.is_inf(), p, r);
-}
-
-// add-2008-s, four levels of products
-template <class F>
-CSB_DEV XYZZ<F> xyzz_add_quad(const XYZZ<F>& p, const XYZZ<F>& q) {
-  F U1, U2, S1, S2;
-  quad_mul4(p.X, q.ZZ, q.X, p.ZZ, p.Y, q.ZZZ, q.Y, p.ZZZ, U1, U2, S1, S2);
-  const F P = U2 - U1;
-  const F R = S2 - S1;
-  F PP, RR, Z2, Z3, PPP, Q, ZZ3, ZZZ3, T1, T2, unused;
-  quad_mul4(P, P, R, R, p.ZZ, q.ZZ, p.ZZZ, q.ZZZ, PP, RR, Z2, Z3);
-  quad_mul4(P, PP, U1, PP, Z2, PP, Z3, P, PPP, Q, ZZ3, unused);
-  XYZZ<F> r;
-  r.X = RR - PPP - Q.dbl();
-  quad_mul4(R, Q - r.X, S1, PPP, Z3, PPP, Z3, PPP, T1, T2, ZZZ3, unused);
-  r.Y = T1 - T2;
-  r.ZZ = ZZ3;
-  r.ZZZ = ZZZ3;
-  if (P.is_zero() && !p.is_inf() && !q.is_inf())  // equal or opposite points (rare): no shuffles
-    r = R.is_zero() ? xyzz_dbl(p) : XYZZ<F>::inf();
-  return p.is_inf() ? q : (q.is_inf() ? p : r);
-}
-
-// madd-2008-s, four levels of products
-template <class F>
-CSB_DEV XYZZ<F> xyzz_madd_quad(const XYZZ<F>& p, const Affine<F>& q) {
-  F U2, S2, PP, RR, PPP, Q, ZZ3, T1, T2, ZZZ3, unused;
-  quad_mul4(q.x, p.ZZ, q.y, p.ZZZ, q.x, p.ZZ, q.y, p.ZZZ, U2, S2, unused, unused);
-  const F P = U2 - p.X;
-  const F R = S2 - p.Y;
-  quad_mul4(P, P, R, R, P, P, R, R, PP, RR, unused, unused);
-  quad_mul4(P, PP, p.X, PP, p.ZZ, PP, p.ZZ, PP, PPP, Q, ZZ3, unused);
-  XYZZ<F> r;
-  r.X = RR - PPP - Q.dbl();
-  quad_mul4(R, Q - r.X, p.Y, PPP, p.ZZZ, PPP, p.ZZZ, PPP, T1, T2, ZZZ3, unused);
-  r.Y = T1 - T2;
-  r.ZZ = ZZ3;
-  r.ZZZ = ZZZ3;
-  if (P.is_zero() && !p.is_inf())  // equal or opposite points (rare): no shuffles
-    r = R.is_zero() ? xyzz_mdbl(q) : XYZZ<F>::inf();
-  return p.is_inf() ? XYZZ<F>::from_affine(q) : r;
-}
 
 template <class F>
 CSB_DEV XYZZ<F> xyzz_neg(const XYZZ<F>& p) {
@@ -356,23 +226,6 @@ template <class F>
 CSB_DEV void st_xyzz(uint32_t* p, const XYZZ<F>& a) {
   constexpr int W = FieldWords<F>::value;
   st_field(p, a.X); st_field(p + W, a.Y); st_field(p + 2 * W, a.ZZ); st_field(p + 3 * W, a.ZZZ);
-}
-
-// Quad operations as calls over Fq2: one body per kernel instead of one per use, for kernels
-// that chain many of them, whose inlined copies overflow the register file.
-template <class F>
-__device__ __noinline__ XYZZ<F> xyzz_add_quad_call(const XYZZ<F> p, const XYZZ<F> q) { return xyzz_add_quad(p, q); }
-template <class F>
-__device__ __noinline__ XYZZ<F> xyzz_dbl_quad_call(const XYZZ<F> p) { return xyzz_dbl_quad(p); }
-template <class F>
-CSB_DEV XYZZ<F> add_q(const XYZZ<F>& p, const XYZZ<F>& q) {
-  if constexpr (FieldWords<F>::value == 16) return xyzz_add_quad_call(p, q);
-  else return xyzz_add_quad(p, q);
-}
-template <class F>
-CSB_DEV XYZZ<F> dbl_q(const XYZZ<F>& p) {
-  if constexpr (FieldWords<F>::value == 16) return xyzz_dbl_quad_call(p);
-  else return xyzz_dbl_quad(p);
 }
 
 }  // namespace csb

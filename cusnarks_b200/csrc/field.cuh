@@ -10,6 +10,8 @@
 #pragma once
 #include <cstdint>
 
+#include "modinv.cuh"
+
 namespace csb {
 
 #define CSB_DEV __device__ __forceinline__
@@ -472,81 +474,9 @@ struct Fp {
     return (*this) * o;
   }
 
-  // Montgomery inverse (aR -> a^-1 R; 0 -> 0).  Binary extended Euclid on the integer
-  // x = aR gives x^-1 = a^-1 R^-1; one Montgomery product by R^3 restores a^-1 R.  Used
-  // for the few final affine conversions, where a single thread's latency is what counts.
-  CSB_DEV Fp inv() const {
-    if (is_zero()) return zero();
-    const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
-    uint32_t u[8], v[8], x1[8], x2[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) { u[i] = this->v[i]; v[i] = P[i]; x1[i] = 0; x2[i] = 0; }
-    x1[0] = 1;
-#pragma unroll 1
-    for (int guard = 0; guard < 2048; guard++) {
-      const bool u1 = (u[0] == 1) && ((u[1] | u[2] | u[3] | u[4] | u[5] | u[6] | u[7]) == 0);
-      const bool v1 = (v[0] == 1) && ((v[1] | v[2] | v[3] | v[4] | v[5] | v[6] | v[7]) == 0);
-      if (u1 || v1) break;
-      // (a zero u or v only arises from an unreduced input; the bounded loops end anyway)
-#pragma unroll 1
-      for (int k = 0; k < 256 && (u[0] & 1u) == 0; k++) { shr1(u); half_mod(x1, P); }
-#pragma unroll 1
-      for (int k = 0; k < 256 && (v[0] & 1u) == 0; k++) { shr1(v); half_mod(x2, P); }
-      if (geq(u, v)) { sub8(u, v); sub_mod(x1, x2, P); }
-      else { sub8(v, u); sub_mod(x2, x1, P); }
-    }
-    const bool u1 = (u[0] == 1) && ((u[1] | u[2] | u[3] | u[4] | u[5] | u[6] | u[7]) == 0);
-    Fp r;
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = u1 ? x1[i] : x2[i];
-    return r * r3();
-  }
-
- private:
-  static CSB_DEV void shr1(uint32_t (&a)[8]) {
-#pragma unroll
-    for (int i = 0; i < 7; i++) a[i] = (a[i] >> 1) | (a[i + 1] << 31);
-    a[7] >>= 1;
-  }
-  static CSB_DEV bool geq(const uint32_t (&a)[8], const uint32_t (&b)[8]) {
-#pragma unroll
-    for (int i = 7; i >= 0; i--) {
-      if (a[i] != b[i]) return a[i] > b[i];
-    }
-    return true;
-  }
-  static CSB_DEV void sub8(uint32_t (&a)[8], const uint32_t (&b)[8]) {
-    SUB_CC(a[0], a[0], b[0]); SUBC_CC(a[1], a[1], b[1]); SUBC_CC(a[2], a[2], b[2]);
-    SUBC_CC(a[3], a[3], b[3]); SUBC_CC(a[4], a[4], b[4]); SUBC_CC(a[5], a[5], b[5]);
-    SUBC_CC(a[6], a[6], b[6]); SUBC(a[7], a[7], b[7]);
-  }
-  // x <- x/2 mod p for x < p
-  static CSB_DEV void half_mod(uint32_t (&x)[8], const uint32_t (&P)[8]) {
-    if (x[0] & 1u) {
-      uint32_t c;
-      ADD_CC(x[0], x[0], P[0]); ADDC_CC(x[1], x[1], P[1]); ADDC_CC(x[2], x[2], P[2]);
-      ADDC_CC(x[3], x[3], P[3]); ADDC_CC(x[4], x[4], P[4]); ADDC_CC(x[5], x[5], P[5]);
-      ADDC_CC(x[6], x[6], P[6]); ADDC_CC(x[7], x[7], P[7]); ADDC(c, 0u, 0u);
-      shr1(x);
-      x[7] |= c << 31;
-    } else {
-      shr1(x);
-    }
-  }
-  // x <- x - y mod p for x, y < p
-  static CSB_DEV void sub_mod(uint32_t (&x)[8], const uint32_t (&y)[8], const uint32_t (&P)[8]) {
-    uint32_t br;
-    SUB_CC(x[0], x[0], y[0]); SUBC_CC(x[1], x[1], y[1]); SUBC_CC(x[2], x[2], y[2]);
-    SUBC_CC(x[3], x[3], y[3]); SUBC_CC(x[4], x[4], y[4]); SUBC_CC(x[5], x[5], y[5]);
-    SUBC_CC(x[6], x[6], y[6]); SUBC_CC(x[7], x[7], y[7]); SUBC(br, 0u, 0u);
-    if (br) {
-      ADD_CC(x[0], x[0], P[0]); ADDC_CC(x[1], x[1], P[1]); ADDC_CC(x[2], x[2], P[2]);
-      ADDC_CC(x[3], x[3], P[3]); ADDC_CC(x[4], x[4], P[4]); ADDC_CC(x[5], x[5], P[5]);
-      ADDC_CC(x[6], x[6], P[6]); ADDC(x[7], x[7], P[7]);
-    }
-  }
-
- public:
+  // Montgomery inverse (aR -> a^-1 R; 0 -> 0): the GCD on the integer x = aR gives
+  // x^-1 = a^-1 R^-1, one Montgomery product by R^3 restores a^-1 R.
+  CSB_DEV Fp inv() const;
 };
 
 using Fq = Fp<ModQ>;
@@ -574,6 +504,16 @@ template <class M>
 __device__ __noinline__ Fp<M> fp_mul2_call(Fp<M> a, Fp<M> b, Fp<M> c, Fp<M> d) {
   return Fp<M>::mul2_raw(a, b, c, d);
 }
+
+template <class M>
+__device__ __noinline__ Fp<M> fp_inv_call(Fp<M> a) {
+  const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
+  Fp<M> r;
+  modinv(a.v, P, M::NP0, r.v);
+  return Fp<M>::mul_raw(Fp<M>::r3(), r).canon();
+}
+template <class M>
+CSB_DEV Fp<M> Fp<M>::inv() const { return fp_inv_call<M>(*this); }
 
 // Out of line (CSB_MUL_NOINLINE units) or inlined
 #if defined(CSB_MUL_NOINLINE)

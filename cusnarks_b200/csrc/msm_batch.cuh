@@ -66,23 +66,12 @@ __global__ void k_bscatter(const BatchJob* __restrict__ jobs, uint32_t njobs, ui
   });
 }
 
-// One warp per instance (quad point operations; the warp's 8 quads compute the same):
+// One warp per instance (block i: instance i):
 // sum_j 2^(c j) S_j over its bucket sets (a fixed-base instance has one), affine result.
 template <class F>
-__global__ void k_bfinish(const BatchJob* __restrict__ jobs, uint32_t njobs, const uint32_t* __restrict__ wsum) {
-  constexpr int XW = 4 * FieldWords<F>::value;
-  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= njobs) return;  // whole warps leave together
-  const BatchJob jb = jobs[q];
-  const uint32_t* w = wsum + (size_t)jb.window0 * XW;
-  XYZZ<F> r = ld_xyzz<F>(w + (size_t)(jb.sets - 1) * XW);
-#pragma unroll 1
-  for (int j = (int)jb.sets - 2; j >= 0; j--) {
-#pragma unroll 1
-    for (uint32_t d = 0; d < jb.c; d++) r = xyzz_dbl_quad(r);
-    r = xyzz_add_quad(r, ld_xyzz<F>(w + (size_t)j * XW));
-  }
-  if ((threadIdx.x & 31) == 0) st_affine<F>(jb.out, xyzz_to_affine(r));
+__global__ void __launch_bounds__(32) k_bfinish(const BatchJob* __restrict__ jobs, const uint32_t* __restrict__ wsum) {
+  const BatchJob jb = jobs[blockIdx.x];
+  windows_horner<F>(wsum + (size_t)jb.window0 * 4 * FieldWords<F>::value, (int)jb.sets, (int)jb.c, jb.out);
 }
 
 struct BatchLayout {
@@ -160,12 +149,14 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   const uint64_t resident_threads = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
   const bool latency_mode = ((uint64_t)nb + b.nentries / task_len + 1) * 4 <= resident_threads * 4;
   if (latency_mode)
-    k_accumulate_quad<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets,
-                                                                  partials, b.d_jobs);
+    k_accumulate_group<F><<<sms * 8, 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets, partials, b.d_jobs);
   else
     k_accumulate<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets,
                                                              partials, b.d_jobs);
-  k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  if (latency_mode)
+    k_combine_group<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  else
+    k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(3);
   const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
@@ -173,24 +164,10 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   for (uint32_t g = 0; g < b.ngroups; g++) {
     const BatchGroup& G = b.groups[g];
     const uint32_t B = 1u << (G.c - 1);
-    const uint32_t WR = G.windows;
-    uint32_t nseg = (B + 7) / 8;
-    reduce_level<F>(buckets + (size_t)G.bucket0 * XWD, nullptr, B, nseg, (int)WR, 0, lv_y, lv_z, resident, st);
-    int levels = 1;
-    uint32_t *y = lv_y, *z = lv_z, *y2 = lv_y2, *z2 = lv_z2;
-    while (nseg > kTopSegments) {
-      const uint32_t nnext = (nseg + 7) / 8;
-      reduce_level<F>(y, z, nseg, nnext, (int)WR, levels, y2, z2, resident, st);
-      uint32_t* ty = y; y = y2; y2 = ty;
-      uint32_t* tz = z; z = z2; z2 = tz;
-      nseg = nnext;
-      levels++;
-    }
-    constexpr int WT = WsumThreads<F>::batch;
-    k_window_sum<F, WT><<<WR, WT, 0, st>>>(y, z, nseg, 3 * levels, wsum + (size_t)G.window0 * XWD);
-    note_launch();
+    reduce_buckets<F>(buckets + (size_t)G.bucket0 * XWD, B, G.windows, lv_y, lv_z, lv_y2, lv_z2,
+                      wsum + (size_t)G.window0 * XWD, nullptr, resident, st);
   }
-  k_bfinish<F><<<(32 * b.njobs + 127) / 128, 128, 0, st>>>(b.d_jobs, b.njobs, wsum);
+  k_bfinish<F><<<b.njobs, 32, 0, st>>>(b.d_jobs, wsum);
   note_launch();
   return cudaGetLastError();
 }

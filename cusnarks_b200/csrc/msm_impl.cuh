@@ -6,6 +6,7 @@
 #include "msm.cuh"
 #include "curve.cuh"
 #include "glv.cuh"
+#include "group.cuh"
 #include "scan.cuh"
 #include "runtime.cuh"
 
@@ -380,53 +381,53 @@ __global__ void __launch_bounds__(128, AccMinBlocks<F>::value) k_accumulate(cons
   }
 }
 
-// Latency form of k_accumulate for an MSM too small to fill the GPU: one quad per task, each
-// lane computing one product of each level of the mixed addition (4 product latencies per
-// addition instead of 10).  Same tasks, same results.  The quad operations shuffle across
-// the whole warp, so the 8 quads of a warp step together: each walks the longest of the
-// warp's 8 tasks and keeps its accumulator past its own task's end (tasks are emitted
-// longest first, so neighbours are about as long).
+// Latency form of k_accumulate for an MSM too small to fill the GPU: one group of lanes per
+// task (group.cuh; 4 product latencies per addition instead of 10).  Same tasks, same results.
+// The groups of a warp step together: each walks the longest of the warp's tasks and leaves
+// its sum alone past its own task's end (tasks are emitted longest first, so neighbours are
+// about as long).
 template <class F>
-__global__ void __launch_bounds__(128, AccMinBlocks<F>::value) k_accumulate_quad(
+__global__ void __launch_bounds__(128, 4) k_accumulate_group(
     const Task* __restrict__ tasks, const uint32_t* __restrict__ counters, const uint32_t* __restrict__ entries,
     const uint32_t* __restrict__ points, uint32_t nb, uint32_t* __restrict__ buckets,
     uint32_t* __restrict__ partials, const BatchJob* __restrict__ jobs = nullptr,
     const uint32_t* __restrict__ phix = nullptr) {
-  constexpr int PW = 2 * FieldWords<F>::value;
-  constexpr int XW = 4 * FieldWords<F>::value;
-  constexpr uint32_t G = GroupLanes<F>::value, QPW = 32 / G;  // lanes per group, groups per warp
+  using Gr = Group<F>;
+  constexpr int FW = FieldWords<F>::value, PW = 2 * FW, XW = 4 * FW;
+  constexpr uint32_t G = Gr::G, GPW = 32 / G, NG = 128 / G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const Gr grp(scr[threadIdx.x / G]);
+  uint32_t* acc = accs[threadIdx.x / G];
   const uint32_t ntasks = counters[0];
   const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t qw = (threadIdx.x & 31) / G;  // group within the warp
-  for (uint32_t base = warp0 * QPW; base < ntasks; base += nwarps * QPW) {  // warp-uniform
-    const uint32_t t = base + qw;
+  const uint32_t gw = (threadIdx.x & 31) / G;  // group within the warp
+  for (uint32_t first = warp0 * GPW; first < ntasks; first += nwarps * GPW) {  // warp-uniform
+    const uint32_t t = first + gw;
     const bool valid = t < ntasks;
     const Task tk = valid ? tasks[t] : Task{0, 0, 0, 0};
     const uint32_t* pts = jobs && valid ? jobs[tk.job].points : points;  // read only where live
     const uint32_t steps = __reduce_max_sync(0xffffffffu, tk.len);
-    XYZZ<F> acc = XYZZ<F>::inf();
+    grp.load(acc, nullptr, false);
 #pragma unroll 1
     for (uint32_t e = 0; e < steps; e++) {
       const bool live = e < tk.len;
-      Affine<F> p{F::zero(), F::zero()};  // past the task's end: not taken
+      const uint32_t *qx = acc, *qy = acc;  // past the task's end: any readable address
+      bool neg = false;
       if (live) {
-        if (entries) {
-          const uint32_t ent = entries[tk.start + e];
-          p = ld_entry_point<F>(pts, phix, ent);
-          if (ent & NEG_BIT) p.y = p.y.neg();
-        } else {
-          p = ld_affine<F>(pts + (size_t)(tk.start + e) * PW);
-        }
+        const uint32_t ent = entries[tk.start + e];
+        const uint32_t i = ent & ~(NEG_BIT | (phix ? PHI_BIT : 0u));
+        qy = pts + (size_t)i * PW + FW;
+        qx = FW == 8 && phix && (ent & PHI_BIT) ? phix + (size_t)i * FW : pts + (size_t)i * PW;
+        neg = (ent & NEG_BIT) != 0;
       }
-      const XYZZ<F> nxt = xyzz_madd_quad(acc, p);
-      const bool take = live && (entries || !(p.x.is_zero() && p.y.is_zero()));
-      acc = xyzz_select(take, nxt, acc);
+      grp.madd(acc, acc, qx, qy, neg, live);
     }
-    if (valid && (threadIdx.x & (G - 1)) == 0) {
+    if (valid) {
       uint32_t* dst = tk.dst < nb ? buckets + (size_t)tk.dst * XW : partials + (size_t)(tk.dst - nb) * XW;
-      st_xyzz<F>(dst, acc);
+      grp.store(dst, acc);
     }
+    __syncwarp();
   }
 }
 
@@ -461,6 +462,37 @@ __global__ void __launch_bounds__(128) k_combine_small(const Multi* __restrict__
 #pragma unroll 1
     for (uint32_t i = 1; i < mu.count; i++) acc = xyzz_add(acc, ld_xyzz<F>(partials + (size_t)(mu.pbase + i) * XW));
     st_xyzz<F>(buckets + (size_t)mu.bucket * XW, acc);
+  }
+}
+
+// k_combine_small with one group of lanes per split bucket (the latency form's).
+template <class F>
+__global__ void __launch_bounds__(128, 4) k_combine_group(const Multi* __restrict__ multi,
+                                                       const uint32_t* __restrict__ counters,
+                                                       const uint32_t* __restrict__ partials,
+                                                       uint32_t* __restrict__ buckets) {
+  using Gr = Group<F>;
+  constexpr int XW = 4 * FieldWords<F>::value;
+  constexpr uint32_t G = Gr::G, GPW = 32 / G, NG = 128 / G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const Gr grp(scr[threadIdx.x / G]);
+  uint32_t* acc = accs[threadIdx.x / G];
+  const uint32_t nm = counters[2];
+  const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t first = warp0 * GPW; first < nm; first += nwarps * GPW) {  // warp-uniform
+    const uint32_t m = first + (threadIdx.x & 31) / G;
+    Multi mu = m < nm ? multi[m] : Multi{0, 0, 0, 0};
+    if (mu.count > kCombineSerial) mu.count = 0;  // k_combine
+    const uint32_t steps = __reduce_max_sync(0xffffffffu, mu.count);
+    grp.load(acc, partials + (size_t)mu.pbase * XW, mu.count != 0);
+#pragma unroll 1
+    for (uint32_t i = 1; i < steps; i++) {
+      const bool live = i < mu.count;
+      grp.add(acc, acc, live ? partials + (size_t)(mu.pbase + i) * XW : acc, live);
+    }
+    if (mu.count) grp.store(buckets + (size_t)mu.bucket * XW, acc);
+    __syncwarp();
   }
 }
 
@@ -550,241 +582,125 @@ __global__ void __launch_bounds__(128) k_reduce_level(const uint32_t* __restrict
 }
 
 
-// k_reduce_level with one quad per output segment (quad point operations): the latency form
-// for levels too small to fill the GPU.  Every lane of a launched warp runs the operations
-// (quads past the end work on points at infinity and store nothing).
-template <class F>
-__global__ void __launch_bounds__(128) k_reduce_level_quad(const uint32_t* __restrict__ y,
-                                                           const uint32_t* __restrict__ z, uint32_t n,
-                                                           uint32_t nout, int W, int level,
-                                                           uint32_t* __restrict__ yout,
-                                                           uint32_t* __restrict__ zout) {
-  constexpr int XW = 4 * FieldWords<F>::value;
-  constexpr uint32_t G = GroupLanes<F>::value;
-  const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const bool valid = g < (uint32_t)W * nout;
-  const uint32_t j = valid ? g / nout : 0u, t = valid ? g % nout : 0u;
-  const uint32_t* yj = y + (size_t)j * n * XW;
-  // running sum acc and sum of running sums s over the segment's buckets 7..1, starting at
-  // bucket 7 (no additions to infinity)
-  XYZZ<F> acc = valid && 8 * t + 7 < n ? ld_xyzz<F>(yj + (size_t)(8 * t + 7) * XW) : XYZZ<F>::inf();
-  XYZZ<F> s = acc;
-#pragma unroll 1
-  for (int i = 6; i >= 1; i--) {
-    const uint32_t idx = 8 * t + i;
-    const XYZZ<F> v = valid && idx < n ? ld_xyzz<F>(yj + (size_t)idx * XW) : XYZZ<F>::inf();
-    acc = add_q(acc, v);
-    s = add_q(s, acc);
-  }
-  {
-    const XYZZ<F> v = valid && 8 * t < n ? ld_xyzz<F>(yj + (size_t)(8 * t) * XW) : XYZZ<F>::inf();
-    acc = add_q(acc, v);
-  }
-#pragma unroll 1
-  for (int d = 0; d < 3 * level; d++) s = dbl_q(s);
-  if (z) {  // uniform: a kernel argument
-    const uint32_t* zj = z + (size_t)j * n * XW;
-#pragma unroll 1
-    for (int i = 0; i < 8; i++) {
-      const uint32_t idx = 8 * t + i;
-      const XYZZ<F> v = valid && idx < n ? ld_xyzz<F>(zj + (size_t)idx * XW) : XYZZ<F>::inf();
-      s = add_q(s, v);
-    }
-  }
-  if (valid && (threadIdx.x & (G - 1)) == 0) {
-    st_xyzz<F>(yout + ((size_t)j * nout + t) * XW, acc);
-    st_xyzz<F>(zout + ((size_t)j * nout + t) * XW, s);
-  }
-}
+// Bucket reduction of few buckets, by bits: with S_b the n = 2^k values of a window (n values of
+// the last level), sum_b b S_b = sum_j 2^j T_j, T_j the sum of the S_b whose index has bit j set.
+// A binary tree gives all T_j at once: joining the left and right halves of a node adds their
+// totals and their T_j pairwise, and the right half's total is the node's new T_j, so 2n
+// additions in all and a chain of k of them, where running sums over segments of eight take
+// about as many additions but chains of 13 a level and a scan over the segments left.
+// One block joins 2^lg <= 64 values in shared memory: node i of level q starts at slot i 2^q and
+// its T_j lies in slot i 2^q + 2^j, where the right half's total already is.  It writes its total
+// and T_j back to the same places, so a later stage finds the earlier bits' partial sums at the
+// same offsets of every 64 slots and adds them up (blockIdx.x: segment and window; blockIdx.y: 0 the totals, which give the
+// next bits; 1..bits the T_j; then z, whose plain sum is needed); after the last stage window w
+// has its total in slot 0 and T_j in slot 2^j.
+// Measured against the segment sums it replaces (group operations there too): see
+// reduce_buckets.
+template <class F> struct TreeGroups { static constexpr int value = 32; };
+template <> struct TreeGroups<Fq2> { static constexpr int value = 16; };  // 48 KB of shared memory
 
 template <class F>
-CSB_DEV XYZZ<F> shfl_down_xyzz(const XYZZ<F>& v, int d) {
+__global__ void __launch_bounds__(Group<F>::G* TreeGroups<F>::value, 512 / (Group<F>::G * TreeGroups<F>::value)) k_bit_tree(uint32_t* __restrict__ y,
+                                                                               uint32_t* __restrict__ z, uint32_t n,
+                                                                               int bits, int lg) {
+  using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
-  XYZZ<F> o;
-  uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-  const uint32_t* vw = reinterpret_cast<const uint32_t*>(&v);
-#pragma unroll
-  for (int w = 0; w < XW; w++) ow[w] = __shfl_down_sync(0xffffffffu, vw[w], d);
-  return o;
-}
-
-// k_reduce_level_quad for the levels that carry weighted sums z (levels >= 1): two quads per
-// output segment, side by side in one warp.  The even quad runs the running sums of the segment
-// totals y and then the doublings; the odd quad sums the segment's eight z values meanwhile (each
-// step is the same point addition on operands picked by role, so the warp does not diverge), and
-// one shuffle and one addition join them: 13 + 3L + 1 dependent point operations instead of
-// 13 + 3L + 8.  Same sums as k_reduce_level_quad.
-template <class F>
-__global__ void __launch_bounds__(128) k_reduce_level_quad2(const uint32_t* __restrict__ y,
-                                                            const uint32_t* __restrict__ z, uint32_t n,
-                                                            uint32_t nout, int W, int level,
-                                                            uint32_t* __restrict__ yout,
-                                                            uint32_t* __restrict__ zout) {
-  constexpr int XW = 4 * FieldWords<F>::value;
-  constexpr uint32_t G = GroupLanes<F>::value;
-  const uint32_t gq = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const uint32_t g = gq >> 1;
-  const bool zq = (gq & 1) != 0;  // the odd quad of the pair sums the z values
-  const bool valid = g < (uint32_t)W * nout;
-  const uint32_t j = valid ? g / nout : 0u, t = valid ? g % nout : 0u;
-  const uint32_t* yj = y + (size_t)j * n * XW;
-  const uint32_t* zj = z + (size_t)j * n * XW;
-  auto ld = [&](const uint32_t* base, uint32_t i) {
-    const uint32_t idx = 8 * t + i;
-    return valid && idx < n ? ld_xyzz<F>(base + (size_t)idx * XW) : XYZZ<F>::inf();
-  };
-  // even quad: a = running sum from bucket 7 down, s = sum of the running sums 7..1;
-  // odd quad: a = z_0 + ... + z_7
-  XYZZ<F> a = zq ? ld(zj, 0) : ld(yj, 7);
-  XYZZ<F> s = a;
-#pragma unroll 1
-  for (int step = 0; step < 13; step++) {
-    // even quad: even steps a += y_i (i = 6..0), odd steps s += a; odd quad: a += z_{step+1}
-    const bool even_step = (step & 1) == 0;
-    XYZZ<F> p, q;
-    if (zq) {
-      p = a;
-      q = step < 7 ? ld(zj, step + 1) : XYZZ<F>::inf();
-    } else if (even_step) {
-      p = a;
-      q = ld(yj, 6 - (step >> 1));
-    } else {
-      p = s;
-      q = a;
-    }
-    const XYZZ<F> r = add_q(p, q);  // every lane of the warp, every step
-    if (zq || even_step) a = r; else s = r;
+  constexpr uint32_t NG = TreeGroups<F>::value, G = Gr::G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], node[64][XW];
+  const Gr grp(scr[threadIdx.x / G]);
+  const uint32_t g = threadIdx.x / G, g0 = (threadIdx.x & ~31u) / G;  // this group, the warp's first
+  const int role = blockIdx.y;
+  const uint32_t segs = n >> (bits + lg), seg = blockIdx.x % segs;
+  uint32_t* arr = (role <= bits ? y : z) + (size_t)(blockIdx.x / segs) * n * XW;
+  const uint32_t off = role >= 1 && role <= bits ? 1u << (role - 1) : 0u;
+  auto at = [&](uint32_t i) { return arr + ((size_t)((((seg << lg) + i) << bits) + off)) * XW; };
+  for (uint32_t w = threadIdx.x; w < (XW / 4u) << lg; w += blockDim.x) {
+    const uint32_t i = w / (XW / 4), q = w % (XW / 4);
+    reinterpret_cast<uint4*>(node[i])[q] = reinterpret_cast<const uint4*>(at(i))[q];
   }
-  // the odd quads double their own s too and drop it: the quad operations shuffle across
-  // the whole warp, so every lane takes part in the same steps (no extra latency)
-#pragma unroll 1
-  for (int d = 0; d < 3 * level; d++) s = dbl_q(s);
-  s = add_q(s, shfl_down_xyzz(a, G));  // even groups: + the odd neighbour's z sum
-  if (valid && !zq && (threadIdx.x & (G - 1)) == 0) {
-    st_xyzz<F>(yout + ((size_t)j * nout + t) * XW, a);
-    st_xyzz<F>(zout + ((size_t)j * nout + t) * XW, s);
-  }
-}
-
-// Per-window sum after levels 0..L-1.  With y_t the segment totals and z_t the weighted
-// carries of the last level, S_j = sum_t (y_t + z_t) + G * sum_t t * y_t with G = 8^L =
-// 2^shift.  One block per window, E consecutive segments per virtual thread u:
-//   V_u = Y_u + Z_u + G * sum_i i*y_{uE+i}      (Y_u, Z_u: the thread's totals)
-//   sum_t t*y_t = sum_u [sum_i i*y_{uE+i}] + E * sum_{u>=1} Suf(u),  Suf(u) = sum_{v>=u} Y_v
-// so S_j = sum_u (Y_u + Z_u + G (W_u + E Suf(u) [u >= 1])) with W_u = sum_i i*y_{uE+i}: a suffix
-// scan and a reduction over the block's virtual threads, about 3E + 2 log2(VT) + shift
-// dependent point operations instead of a serial pass over the segments.
-// Threads of the per-window sum (one block per window).  128 (4 warps, one per SM
-// sub-partition) shortens each dependent point operation enough to pay for the longer chains
-// of 32 virtual threads: 2^12 proof 2.00 -> 1.91 ms, G2 2^12 fixed-base MSM 1.68 -> 1.58 ms.
-// Over Fq2 (16-lane groups) 256 threads, 16 virtual threads, for the single MSM and batches
-// (128: G2 fixed-base 2^20 13.5 ms, 256: 13.0; 512 slower at every size).
-constexpr int kWsumThreads = 128;
-template <class F> struct WsumThreads { static constexpr int single = kWsumThreads, batch = 256; };
-template <> struct WsumThreads<Fq2> { static constexpr int single = 256, batch = 256; };
-template <class F, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_window_sum(const uint32_t* __restrict__ y,
-                                                        const uint32_t* __restrict__ z, uint32_t n1,
-                                                        int shift, uint32_t* __restrict__ wsum) {
-  // Group form: each group of G lanes is one virtual thread u running group point operations,
-  // so the block has VT = THREADS / G virtual threads.  The scan and the reduction across them
-  // go through shared memory (double-buffered Hillis-Steele steps); the group's first lane
-  // writes, every lane reads.
-  constexpr int XW = 4 * FieldWords<F>::value;
-  constexpr uint32_t G = GroupLanes<F>::value;
-  constexpr uint32_t VT = THREADS / G;
-  static_assert(VT >= 1 && (VT & (VT - 1)) == 0, "virtual threads: a power of two");
-  __shared__ uint32_t sh[2][VT][XW];
-  const int j = blockIdx.x;
-  const uint32_t* yj = y + (size_t)j * n1 * XW;
-  const uint32_t* zj = z + (size_t)j * n1 * XW;
-  const uint32_t E = (n1 + VT - 1) / VT;  // n1 is a power of two
-  const uint32_t u = threadIdx.x / G;
-  const bool lead = (threadIdx.x & (G - 1)) == 0;
-  auto put = [&](int b, uint32_t slot, const XYZZ<F>& v) {
-    if (lead) {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
-      for (int k = 0; k < XW; k++) sh[b][slot][k] = w[k];
-    }
-  };
-  auto get = [&](int b, uint32_t slot) {
-    XYZZ<F> v;
-    uint32_t* w = reinterpret_cast<uint32_t*>(&v);
-    for (int k = 0; k < XW; k++) w[k] = sh[b][slot][k];
-    return v;
-  };
-  // the sums start at the thread's last segment (no additions to infinity)
-  XYZZ<F> acc, zs, ws = XYZZ<F>::inf();
-  {
-    const uint32_t idx = u * E + (E - 1);
-    const bool in = idx < n1;
-    acc = in ? ld_xyzz<F>(yj + (size_t)idx * XW) : XYZZ<F>::inf();
-    zs = in ? ld_xyzz<F>(zj + (size_t)idx * XW) : XYZZ<F>::inf();
-  }
-#pragma unroll 1
-  for (int i = (int)E - 2; i >= 0; i--) {  // uniform trip count; past n1 the terms are infinity
-    const uint32_t idx = u * E + i;
-    const bool in = idx < n1;
-    ws = add_q(ws, acc);  // acc = sum of the thread's segments above i
-    acc = add_q(acc, in ? ld_xyzz<F>(yj + (size_t)idx * XW) : XYZZ<F>::inf());
-    zs = add_q(zs, in ? ld_xyzz<F>(zj + (size_t)idx * XW) : XYZZ<F>::inf());
-  }
-  // V_u = acc + zs + 2^shift (ws + E Suf(u) [u >= 1]): one chain of shift doublings for both
-  // terms (ws is infinity with one segment per thread)
-  XYZZ<F> V = add_q(acc, zs);
-  // inclusive suffix scan of acc over the virtual threads: Suf(u)
-  XYZZ<F> suf = acc;
-  int cur = 0;
-  put(cur, u, suf);
   __syncthreads();
-#pragma unroll 1
-  for (uint32_t d = 1; d < VT; d <<= 1) {
-    const bool has = u + d < VT;
-    const XYZZ<F> o = has ? get(cur, u + d) : XYZZ<F>::inf();
-    suf = xyzz_select(has, add_q(suf, o), suf);
-    cur ^= 1;
-    put(cur, u, suf);
+  for (int q = 1; q <= lg; q++) {
+    const uint32_t half = 1u << (q - 1), per = role == 0 ? (uint32_t)q : 1u;
+    const uint32_t ops = (1u << (lg - q)) * per;
+    for (uint32_t o0 = 0; o0 + g0 < ops; o0 += NG) {  // warp-uniform
+      const uint32_t o = o0 + g;
+      const bool live = o < ops;
+      const uint32_t i = live ? o / per : 0u, k = live ? o % per : 0u;  // k: 0 the total, k - 1 the bit
+      const uint32_t dst = (i << q) + (k ? 1u << (k - 1) : 0u);
+      grp.add(node[dst], node[dst], node[dst + half], live);
+    }
     __syncthreads();
   }
-  {  // computed by every group (uniform); E Suf(u) kept where u >= 1 and u E < n1
-#pragma unroll 1
-    for (uint32_t m = E; m > 1; m >>= 1) suf = dbl_q(suf);  // E is a power of two
-    XYZZ<F> T = xyzz_select(u >= 1 && u * E < n1, add_q(ws, suf), ws);
-#pragma unroll 1
-    for (int d = 0; d < shift; d++) T = dbl_q(T);
-    V = add_q(V, T);
+  const uint32_t outs = role == 0 ? (uint32_t)lg + 1 : 1u;
+  for (uint32_t o = g; o < outs; o += NG) {
+    const uint32_t i = o ? 1u << (o - 1) : 0u;
+    grp.store(at(i), node[i]);
   }
-  // reduction of V over the virtual threads
-  cur ^= 1;  // the buffer no step reads any more
-  put(cur, u, V);
-  __syncthreads();
+}
+
+// One warp per window: Z + Y + 2^shift sum_j 2^j T_j from the places k_bit_tree left them in (z
+// null: no Z), the bits in two halves at once: the upper half's Horner chain, doubled over the
+// lower bits, joins the lower's.  out: the affine result (one window), else wsum[window].
+template <class F>
+__global__ void __launch_bounds__(32) k_window_horner(const uint32_t* __restrict__ y, const uint32_t* __restrict__ z,
+                                                      uint32_t n, int bits, int shift, uint32_t* __restrict__ wsum,
+                                                      uint32_t* __restrict__ out) {
+  using Gr = Group<F>;
+  constexpr int XW = 4 * FieldWords<F>::value;
+  constexpr uint32_t G = Gr::G, NG = 32 / G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const Gr grp(scr[threadIdx.x / G]);
+  uint32_t* acc = accs[threadIdx.x / G];
+  const bool upper = ((threadIdx.x / G) & 1) != 0;
+  const uint32_t* yw = y + (size_t)blockIdx.x * n * XW;
+  const int s = (bits + 1) / 2, lo = upper ? s : 0;
+  auto has = [&](int i) { return lo + i < bits; };
+  auto T = [&](int i) { return yw + ((size_t)1 << (lo + i)) * XW; };
+  grp.load(acc, s > 0 ? T(s - 1) : yw, s > 0 && has(s - 1));
 #pragma unroll 1
-  for (uint32_t d = VT / 2; d >= 1; d >>= 1) {
-    const bool has = u < d;
-    const XYZZ<F> o = has ? get(cur, u + d) : XYZZ<F>::inf();
-    V = xyzz_select(has, add_q(V, o), V);
-    cur ^= 1;
-    put(cur, u, V);
-    __syncthreads();
+  for (int i = s - 2; i >= 0; i--) {
+    grp.dbl(acc, acc);
+    grp.add(acc, acc, has(i) ? T(i) : acc, has(i));
   }
-  if (u == 0 && lead) st_xyzz<F>(wsum + (size_t)j * XW, V);
+#pragma unroll 1
+  for (int i = 0; i < s; i++) grp.dbl(acc, acc, upper);
+  uint32_t* a0 = accs[0];
+  grp.add(acc, acc, accs[(threadIdx.x / G) | 1], !upper);
+#pragma unroll 1
+  for (int i = 0; i < shift; i++) grp.dbl(acc, acc);
+  grp.add(acc, acc, yw, !upper);
+  if (z) grp.add(acc, acc, z + (size_t)blockIdx.x * n * XW, !upper);
+  if (threadIdx.x >= G) return;
+  if (out) {
+    if (threadIdx.x == 0) Gr::store_affine(out, a0);
+  } else {
+    grp.store(wsum + (size_t)blockIdx.x * XW, a0);
+  }
 }
 
 // sum_j 2^(c j) S_j (Horner over the windows) and the affine result.
 template <class F>
-__global__ void k_finish(const uint32_t* __restrict__ wsum, int W, int c, uint32_t* __restrict__ out) {
+CSB_DEV void windows_horner(const uint32_t* wsum, int W, int c, uint32_t* out) {
+  // one warp; its groups compute the same
+  using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
-  if (blockIdx.x != 0) return;
-  // one warp (launched with 32 threads; its 8 quads compute the same): the independent
-  // products of each doubling and addition run on the lanes of a quad
-  XYZZ<F> r = ld_xyzz<F>(wsum + (size_t)(W - 1) * XW);
+  constexpr uint32_t G = Gr::G, NG = 32 / G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const Gr grp(scr[(threadIdx.x & 31) / G]);
+  uint32_t* acc = accs[(threadIdx.x & 31) / G];
+  grp.load(acc, wsum + (size_t)(W - 1) * XW);
 #pragma unroll 1
   for (int j = W - 2; j >= 0; j--) {
 #pragma unroll 1
-    for (int d = 0; d < c; d++) r = xyzz_dbl_quad(r);
-    r = xyzz_add_quad(r, ld_xyzz<F>(wsum + (size_t)j * XW));
+    for (int d = 0; d < c; d++) grp.dbl(acc, acc);
+    grp.add(acc, acc, wsum + (size_t)j * XW);
   }
-  if (threadIdx.x == 0) st_affine<F>(out, xyzz_to_affine(r));
+  if ((threadIdx.x & 31) == 0) Gr::store_affine(out, acc);
+}
+template <class F>
+__global__ void __launch_bounds__(32) k_finish(const uint32_t* __restrict__ wsum, int W, int c,
+                                               uint32_t* __restrict__ out) {
+  windows_horner<F>(wsum, W, c, out);
 }
 
 template <class F>
@@ -956,8 +872,9 @@ static __global__ void k_half_counts(const uint32_t* __restrict__ off, uint32_t 
 constexpr int kCtrHist = 16, kCtrCursor = 128, kCtrWords = 256;
 static_assert(kCtrHist + kMaxTask + 1 <= kCtrCursor && kCtrCursor + kMaxTask + 1 <= kCtrWords,
               "task-length bins must not overlap");
-// the reduction adds levels until a window has at most this many segments
-constexpr uint32_t kTopSegments = 256;
+// the reduction runs eight buckets per thread while the remaining values times a group's lanes
+// exceed this many times the resident threads
+constexpr uint64_t kTreeFill = 4;
 
 struct Layout {
   size_t counts, offsets, entries, tasks, multi, partials, buckets, lv_y, lv_z, lv_y2, lv_z2, wsum,
@@ -1066,25 +983,33 @@ int accumulate_grid(int dev, int sms) {
   return b * sms;
 }
 
-// One level of the bucket reduction (level 0: y = the buckets, z = null): one thread per
-// output segment while the level's groups would not fit the resident threads (least work,
-// for full GPUs), else one group per segment (group point operations: a fraction of the
-// chain's latency for a little more work).
+// The window sums of WR bucket sets of B = 2^(c-1) buckets each (overwritten), to wsum, or the
+// affine result of a single set to out.  Levels of eight buckets per thread (least work) while
+// the rest would fill the resident threads' groups several times over, then the bit tree.
 template <class F>
-void reduce_level(const uint32_t* y, const uint32_t* z, uint32_t n, uint32_t nout, int W, int level,
-                  uint32_t* yout, uint32_t* zout, uint64_t resident, cudaStream_t st) {
-  const uint64_t outs = (uint64_t)W * nout;
-  // group forms while their lanes fit the resident threads once (G lanes per point
-  // operation: 4 over Fq, 16 over Fq2); letting 16-lane groups run up to four times over
-  // slowed a 2^20 proof 26.0 -> 26.8 ms and a batch of 16 proofs of 2^12 3.57 -> 3.94 ms
-  constexpr uint64_t G = GroupLanes<F>::value;
-  if (z && outs * 2 * G <= resident)
-    k_reduce_level_quad2<F><<<(uint32_t)((outs * 2 * G + 127) / 128), 128, 0, st>>>(y, z, n, nout, W, level, yout,
-                                                                                   zout);
-  else if (outs * G <= resident)
-    k_reduce_level_quad<F><<<(uint32_t)((outs * G + 127) / 128), 128, 0, st>>>(y, z, n, nout, W, level, yout, zout);
-  else
-    k_reduce_level<F><<<(uint32_t)((outs + 127) / 128), 128, 0, st>>>(y, z, n, nout, W, level, yout, zout);
+void reduce_buckets(uint32_t* buckets, uint32_t B, uint32_t WR, uint32_t* lv_y, uint32_t* lv_z, uint32_t* lv_y2,
+                    uint32_t* lv_z2, uint32_t* wsum, uint32_t* out, uint64_t resident, cudaStream_t st) {
+  uint32_t *y = buckets, *z = nullptr, n = B;
+  int level = 0;
+  while (n >= 8 && (uint64_t)n * WR * Group<F>::G > kTreeFill * resident) {
+    const uint32_t nout = n / 8;
+    uint32_t *yo = level % 2 ? lv_y2 : lv_y, *zo = level % 2 ? lv_z2 : lv_z;
+    k_reduce_level<F><<<(uint32_t)(((uint64_t)WR * nout + 127) / 128), 128, 0, st>>>(y, z, n, nout, (int)WR, level, yo, zo);
+    note_launch();
+    y = yo;
+    z = zo;
+    n = nout;
+    level++;
+  }
+  int k = 0;
+  while ((1u << k) < n) k++;
+  for (int bits = 0; bits < k; bits += 6) {
+    const int lg = std::min(6, k - bits);
+    k_bit_tree<F><<<dim3(WR * (n >> (bits + lg)), 1 + bits + (z ? 1 : 0)), Group<F>::G * TreeGroups<F>::value, 0, st>>>(
+        y, z, n, bits, lg);
+    note_launch();
+  }
+  k_window_horner<F><<<WR, 32, 0, st>>>(y, z, n, k, 3 * level, wsum, out);
   note_launch();
 }
 
@@ -1227,13 +1152,16 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
   note_launch();
   if (cfg.acc_start) cudaEventRecord(cfg.acc_start, st);
   if (latency_mode)
-    k_accumulate_quad<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, acc_entries, acc_points, nb,
-                                                                  buckets, partials, nullptr, phix);
+    k_accumulate_group<F><<<sms * 8, 128, 0, st>>>(tasks, counters, acc_entries, acc_points, nb, buckets, partials,
+                                                    nullptr, phix);
   else
     k_accumulate<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, acc_entries, acc_points, nb,
                                                              buckets, partials, nullptr, phix);
   note_launch();
-  k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  if (latency_mode)
+    k_combine_group<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  else
+    k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(2);
   if (cfg.acc_stop) cudaEventRecord(cfg.acc_stop, st);
@@ -1249,25 +1177,11 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
     k_add_buckets<F><<<(B + 127) / 128, 128, 0, st>>>(buckets, cfg.bucket_add, B);
     note_launch();
   }
-  // level 0: segments of 8 buckets -> totals y and in-segment weighted sums z
-  uint32_t nseg = (B + 7) / 8;
-  reduce_level<F>(buckets, nullptr, B, nseg, WR, 0, lv_y, lv_z, resident, st);
-  int levels = 1;
-  uint32_t *y = lv_y, *z = lv_z, *y2 = lv_y2, *z2 = lv_z2;
-  // more levels until the top block's chain is short
-  while (nseg > kTopSegments) {
-    const uint32_t nnext = (nseg + 7) / 8;
-    reduce_level<F>(y, z, nseg, nnext, WR, levels, y2, z2, resident, st);
-    uint32_t* ty = y; y = y2; y2 = ty;
-    uint32_t* tz = z; z = z2; z2 = tz;
-    nseg = nnext;
-    levels++;
+  reduce_buckets<F>(buckets, B, (uint32_t)WR, lv_y, lv_z, lv_y2, lv_z2, wsum, WR == 1 ? d_out : nullptr, resident, st);
+  if (WR > 1) {
+    k_finish<F><<<1, 32, 0, st>>>(wsum, WR, c, d_out);
+    note_launch();
   }
-  constexpr int WT = WsumThreads<F>::single;
-  k_window_sum<F, WT><<<WR, WT, 0, st>>>(y, z, nseg, 3 * levels, wsum);
-  note_launch();
-  k_finish<F><<<1, 32, 0, st>>>(wsum, WR, c, d_out);
-  note_launch();
   return cudaGetLastError();
 }
 

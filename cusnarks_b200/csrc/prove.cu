@@ -29,6 +29,7 @@
 #include "msm.cuh"
 #include "ntt.cuh"
 #include "glv.cuh"
+#include "group.cuh"
 #include "qap.cuh"
 #include "runtime.cuh"
 
@@ -145,52 +146,81 @@ inline GlvSplit split(const uint32_t* k32) {
 }
 }  // namespace glv_host
 
-// out (XYZZ) = k * P for P affine (G1), k given as its GLV split.
-// One warp (launched with 32 threads; its 8 quads compute the same): the independent
-// products of each doubling and addition run on the lanes of a quad; lane 0 stores.
+// out (XYZZ) = k * P for P affine (G1), k given as its GLV split: k P = k1 P + phi(k2 P).
+// One block of 128 threads, 32 groups of lanes (group.cuh).  The 127 doublings 2^i P are one
+// chain (its first warp); the sums over the set bits of k1 and k2 are not: 16 groups each add
+// up 8 of the 2^i P, a tree joins them, and phi and the signs come last: 435 dependent
+// products instead of the 760 of a joint double-and-add.
+constexpr int kScaleThreads = 128;
 __device__ void scale_point_glv(const uint32_t* __restrict__ P, const GlvSplit* __restrict__ gs,
                                 uint32_t* __restrict__ out) {
-  Fq beta;
-  glv::beta_mont(beta.v);
-  const GlvSplit g = *gs;
-  Affine<Fq> p = ld_affine<Fq>(P);
-  XYZZ<Fq> acc = XYZZ<Fq>::inf();
-  if (!affine_is_inf(p)) {
-    Affine<Fq> q{p.x * beta, p.y};  // phi(P) = lambda P
-    if (g.neg1) p.y = p.y.neg();
-    if (g.neg2) q.y = q.y.neg();
-    const XYZZ<Fq> pq = xyzz_madd(XYZZ<Fq>::from_affine(p), q);  // P + phi(P) (never infinity)
-    for (int b = 127; b >= 0; b--) {
-      acc = xyzz_dbl_quad(acc);
-      const uint32_t e1 = (g.k1[b >> 5] >> (b & 31)) & 1u, e2 = (g.k2[b >> 5] >> (b & 31)) & 1u;
-      if (e1 && e2) acc = xyzz_add_quad(acc, pq);
-      else if (e1) acc = xyzz_add_quad(acc, XYZZ<Fq>::from_affine(p));
-      else if (e2) acc = xyzz_add_quad(acc, XYZZ<Fq>::from_affine(q));
+  using Gr = Group<Fq>;
+  __shared__ __align__(16) uint32_t scr[32][Gr::kScratch], pw[128][32], acc[32][32];
+  const uint32_t g = threadIdx.x / Gr::G;
+  const Gr grp(scr[g]);
+  if (threadIdx.x < 32) {  // 2^i P (every group of the warp computes and stores the same)
+    const Affine<Fq> p = ld_affine<Fq>(P);
+    const XYZZ<Fq> x = affine_is_inf(p) ? XYZZ<Fq>::inf() : XYZZ<Fq>::from_affine(p);
+    if (threadIdx.x == 0) {
+      sts_fq(pw[0], x.X); sts_fq(pw[0] + 8, x.Y); sts_fq(pw[0] + 16, x.ZZ); sts_fq(pw[0] + 24, x.ZZZ);
     }
+    __syncwarp();
+#pragma unroll 1
+    for (int i = 1; i < 128; i++) grp.dbl(pw[i], pw[i - 1], g == 0);
   }
-  if (threadIdx.x == 0) st_xyzz<Fq>(out, acc);
+  __syncthreads();
+  const uint32_t half = g >> 4, b0 = 8 * (g & 15);
+  const uint32_t bits = ((half ? gs->k2 : gs->k1)[b0 >> 5] >> (b0 & 31)) & 0xffu;
+  grp.load(acc[g], nullptr, false);
+#pragma unroll 1
+  for (int i = 0; i < 8; i++) grp.add(acc[g], acc[g], pw[b0 + i], ((bits >> i) & 1u) != 0);
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t d = 8; d >= 1; d >>= 1) {
+    grp.add(acc[g], acc[g], acc[(g & 16) | ((g + d) & 15)], (g & 15) < d);
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+    // the signs, and phi(x, y) = (beta x, y) on the k2 half
+    if (threadIdx.x == 0) {
+      Fq beta;
+      glv::beta_mont(beta.v);
+      if (gs->neg1) sts_fq(acc[0] + 8, Fq::sub_lazy(Fq::zero(), lds_fq(acc[0] + 8)));
+      if (gs->neg2) sts_fq(acc[16] + 8, Fq::sub_lazy(Fq::zero(), lds_fq(acc[16] + 8)));
+      sts_fq(acc[16], Fq::mul_raw(lds_fq(acc[16]), beta));
+    }
+    __syncwarp();
+    grp.add(acc[0], acc[0], acc[16], g == 0);
+    if (g == 0) grp.store(out, acc[0]);
+  }
 }
-__global__ void k_scale_point_glv(const uint32_t* __restrict__ P, const GlvSplit* __restrict__ gs,
-                                  uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(kScaleThreads) k_scale_point_glv(const uint32_t* __restrict__ P,
+                                                                   const GlvSplit* __restrict__ gs,
+                                                                   uint32_t* __restrict__ out) {
   scale_point_glv(P, gs, out);
 }
 
-// pi_C = C2 + C + sA + rB1 (C2, C affine; sA, rB1 XYZZ) -> affine
+// pi_C = C2 + C + sA + rB1 (C2, C affine; sA, rB1 XYZZ) -> affine; one warp (its first group of
+// lanes; the others compute on copies)
 __device__ void final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c,
                         const uint32_t* __restrict__ sa, const uint32_t* __restrict__ rb1,
                         uint32_t* __restrict__ out) {
-  XYZZ<Fq> acc = XYZZ<Fq>::inf();
-  const Affine<Fq> a = ld_affine<Fq>(c2), b = ld_affine<Fq>(c);
-  if (!affine_is_inf(a)) acc = xyzz_madd(acc, a);
-  if (!affine_is_inf(b)) acc = xyzz_madd(acc, b);
-  acc = xyzz_add(acc, ld_xyzz<Fq>(sa));
-  acc = xyzz_add(acc, ld_xyzz<Fq>(rb1));
-  st_affine<Fq>(out, xyzz_to_affine(acc));
+  using Gr = Group<Fq>;
+  __shared__ __align__(16) uint32_t scr[8][Gr::kScratch], accs[8][32];
+  const uint32_t g = (threadIdx.x & 31) / Gr::G;
+  const Gr grp(scr[g]);
+  uint32_t* acc = accs[g];
+  grp.load(acc, nullptr, false);
+  grp.madd(acc, acc, c2, c2 + 8, false, !affine_is_inf(ld_affine<Fq>(c2)));
+  grp.madd(acc, acc, c, c + 8, false, !affine_is_inf(ld_affine<Fq>(c)));
+  grp.add(acc, acc, sa);
+  grp.add(acc, acc, rb1);
+  if ((threadIdx.x & 31) == 0) Gr::store_affine(out, acc);
 }
-__global__ void k_final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c,
-                          const uint32_t* __restrict__ sa, const uint32_t* __restrict__ rb1,
-                          uint32_t* __restrict__ out) {
-  if (threadIdx.x == 0) final_c(c2, c, sa, rb1, out);
+__global__ void __launch_bounds__(32) k_final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c,
+                                                const uint32_t* __restrict__ sa, const uint32_t* __restrict__ rb1,
+                                                uint32_t* __restrict__ out) {
+  final_c(c2, c, sa, rb1, out);
 }
 
 cudaError_t copy_in(void* dst, const void* src, size_t bytes, int on_device, cudaStream_t st) {
@@ -308,8 +338,8 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
   if (P.share_ch && (e = cudaEventRecord(ctx->aux_ev[7], sc)) != cudaSuccess) { *where = "prove C buckets"; return e; }
   {
     const GlvSplit* gsp = reinterpret_cast<const GlvSplit*>(rs + 32);
-    k_scale_point_glv<<<1, 32, 0, sa>>>(outA, gsp, sA);        // s * pi_A
-    k_scale_point_glv<<<1, 32, 0, sb1>>>(outB1, gsp + 1, rB1);  // r * pi_B1
+    k_scale_point_glv<<<1, kScaleThreads, 0, sa>>>(outA, gsp, sA);        // s * pi_A
+    k_scale_point_glv<<<1, kScaleThreads, 0, sb1>>>(outB1, gsp + 1, rB1);  // r * pi_B1
   }
   note_launch(2);
   // QAP evaluation, H step and H MSM on their own stream
@@ -472,8 +502,8 @@ __global__ void k_batch_prep(const BatchCall* __restrict__ calls, uint32_t nv, c
   }
 }
 
-// s pi_A and r pi_B1 of every proof: block 2k + which, one warp each.
-__global__ void k_batch_scale(char* __restrict__ base, size_t per, size_t o_pts, size_t o_rs) {
+// s pi_A and r pi_B1 of every proof: block 2k + which.
+__global__ void __launch_bounds__(kScaleThreads) k_batch_scale(char* __restrict__ base, size_t per, size_t o_pts, size_t o_rs) {
   const uint32_t k = blockIdx.x >> 1, which = blockIdx.x & 1;
   uint32_t* pts = reinterpret_cast<uint32_t*>(base + (size_t)k * per + o_pts);
   const GlvSplit* gs = reinterpret_cast<const GlvSplit*>(base + (size_t)k * per + o_rs + 32 * 4) + which;
@@ -489,9 +519,9 @@ __global__ void k_batch_rs(char* __restrict__ base, size_t per, size_t o_rs, siz
 }
 
 // pi_C of every proof (block k): needs the G1 MSMs, their scalings and the H MSMs, not G2.
-__global__ void k_batch_pic(char* __restrict__ base, size_t per, size_t o_pts) {
+__global__ void __launch_bounds__(32) k_batch_pic(char* __restrict__ base, size_t per, size_t o_pts) {
   uint32_t* pts = reinterpret_cast<uint32_t*>(base + (size_t)blockIdx.x * per + o_pts);
-  if (threadIdx.x == 0) final_c(pts + 80, pts + 64, pts + 96, pts + 128, pts + 160);
+  final_c(pts + 80, pts + 64, pts + 96, pts + 128, pts + 160);
 }
 
 // The proof words of every proof (block k) to the caller's buffer.
@@ -518,7 +548,7 @@ cudaError_t prove_batch_body(cs_ctx* ctx, cs_pk* pk, ProveBatch& B, Domain* dom1
   for (cudaStream_t st : {sa, sb, sh}) cudaStreamWaitEvent(st, ctx->aux_ev[0], 0);
   // A, B1, C of every proof; then the GLV scalings (they read pi_A, pi_B1)
   if ((e = batch_enqueue(B.g1abc, sa)) != cudaSuccess) { *where = "prove batch G1 MSMs"; return e; }
-  k_batch_scale<<<2 * K, 32, 0, sa>>>(base, B.per, B.o_pts, B.o_rs);
+  k_batch_scale<<<2 * K, kScaleThreads, 0, sa>>>(base, B.per, B.o_pts, B.o_rs);
   note_launch();
   if ((e = batch_enqueue(B.g2, sb)) != cudaSuccess) { *where = "prove batch G2 MSMs"; return e; }
   {  // the K QAP evaluations and H steps as batched launches (per-proof arrays B.per bytes apart)
