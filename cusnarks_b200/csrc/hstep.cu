@@ -494,9 +494,25 @@ int cs_hstep_device(cs_ctx* ctx, int variant, const uint32_t* d_A, const uint32_
   if (e == cudaSuccess) e = domain_get(ctx, log_m, &dom1);
   if (e != cudaSuccess) return fail(ctx, e, "hstep domain");
   const size_t mb = (size_t)32 << log_m;
-  if ((e = ctx->work.reserve((variant == CS_HSTEP_COSET ? 6 : 4) * mb, ctx->stream)) != cudaSuccess) return fail(ctx, e, "hstep scratch");
+  // the reference variant's last transform still reads A and B: where the output lies over one
+  // of them they are copied first
+  auto over = [&](const uint32_t* x) {
+    const uintptr_t o = reinterpret_cast<uintptr_t>(d_out), a = reinterpret_cast<uintptr_t>(x);
+    return a < o + 2 * mb && o < a + mb;
+  };
+  const bool copy = variant == CS_HSTEP_REFERENCE && (over(d_A) || over(d_B));
+  if ((e = ctx->work.reserve((variant == CS_HSTEP_COSET || copy ? 6 : 4) * mb, ctx->stream)) != cudaSuccess)
+    return fail(ctx, e, "hstep scratch");
   uint32_t* scr = static_cast<uint32_t*>(ctx->work.ptr);
   cudaEventRecord(ctx->ev_start, ctx->stream);
+  if (copy) {
+    uint32_t* ab = scr + mb;  // past the 4 m elements the core works in (mb bytes, 4 a word)
+    if ((e = cudaMemcpyAsync(ab, d_A, mb, cudaMemcpyDeviceToDevice, ctx->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(ab + mb / 4, d_B, mb, cudaMemcpyDeviceToDevice, ctx->stream)) != cudaSuccess)
+      return fail(ctx, e, "hstep inputs");
+    d_A = ab;
+    d_B = ab + mb / 4;
+  }
   if (variant == CS_HSTEP_REFERENCE)
     e = hstep_reference_core(d_A, d_B, log_m, dom2->Wf, dom2->Wi, dom2->Wf, dom1->consts + 72,
                              dom2->consts + 24, d_out, scr, ctx->stream);

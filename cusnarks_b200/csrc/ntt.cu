@@ -226,15 +226,13 @@ __global__ void k_gather_roots(uint32_t* __restrict__ out, const uint32_t* __res
 }
 
 // Stages per pass.  At least two passes from 2^9 points on: one block would run alone on its
-// SM otherwise (2^11 points 50 us in one pass, 17 in two).  Two passes of equal odd size shift
-// one stage, an even number of stages needs no single one (k_ntt_pass4).
+// SM otherwise (2^11 points 50 us in one pass, 17 in two).
 void plan_passes(uint32_t L, uint32_t* sizes, int* np) {
   const int n = std::max((int)((L + kMaxStages - 1) / kMaxStages), L >= 9 ? 2 : 1);
   int k = 0;
   uint32_t left = L;
   for (int p = 0; p < n; p++) {
-    uint32_t sz = (left + (n - p) - 1) / (n - p);  // even split, larger first
-    if (n == 2 && p == 0 && sz * 2 == L && (sz & 1) && sz < (uint32_t)kMaxStages) sz++;
+    const uint32_t sz = (left + (n - p) - 1) / (n - p);  // even split, larger first
     sizes[k++] = sz;
     left -= sz;
   }
