@@ -436,6 +436,25 @@ struct Fp {
     for (int i = 0; i < 8; i++) r.v[i] = (a.v[i] & br) | (u[i] & ~br);
     return r;
   }
+  // k a mod p, below 2p, for a < 2p and k <= 1024: the 9-limb product less q p, with q from its
+  // top bits (2^238 and up) times 2^270 / p, at most one below the true quotient
+  static CSB_DEV Fp mul_small(const Fp& a, uint32_t k) {
+    constexpr uint32_t kInv = 0x15291u;  // floor(2^270 / p), the same for both moduli
+    const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
+    uint32_t e[8], o[8], t[9];
+    eo_mul(e, o, a.v, k);
+    t[0] = e[0];
+    ADD_CC(t[1], e[1], o[0]);  ADDC_CC(t[2], e[2], o[1]); ADDC_CC(t[3], e[3], o[2]); ADDC_CC(t[4], e[4], o[3]);
+    ADDC_CC(t[5], e[5], o[4]); ADDC_CC(t[6], e[6], o[5]); ADDC_CC(t[7], e[7], o[6]); ADDC(t[8], o[7], 0u);
+    const uint32_t q = __umulhi((t[8] << 18) | (t[7] >> 14), kInv);
+    eo_mul(e, o, P, q);
+    Fp r;
+    SUB_CC(r.v[0], t[0], e[0]);  SUBC_CC(r.v[1], t[1], e[1]); SUBC_CC(r.v[2], t[2], e[2]); SUBC_CC(r.v[3], t[3], e[3]);
+    SUBC_CC(r.v[4], t[4], e[4]); SUBC_CC(r.v[5], t[5], e[5]); SUBC_CC(r.v[6], t[6], e[6]); SUBC(r.v[7], t[7], e[7]);
+    SUB_CC(r.v[1], r.v[1], o[0]);  SUBC_CC(r.v[2], r.v[2], o[1]); SUBC_CC(r.v[3], r.v[3], o[2]);
+    SUBC_CC(r.v[4], r.v[4], o[3]); SUBC_CC(r.v[5], r.v[5], o[4]); SUBC_CC(r.v[6], r.v[6], o[5]); SUBC(r.v[7], r.v[7], o[6]);
+    return r;
+  }
   // zero mod p for a value < 2p: 0 or p
   CSB_DEV bool is_zero_lazy() const {
     const uint32_t z = v[0] | v[1] | v[2] | v[3] | v[4] | v[5] | v[6] | v[7];

@@ -100,7 +100,7 @@ __host__ __device__ inline void modinv(const uint32_t* x, const uint32_t* p, uin
       xb = (uint64_t)b[1] << 32 | b[0];
     }
     int32_t f0 = 1, g0 = 0, f1 = 0, g1 = 1;
-#pragma unroll 1
+#pragma unroll 5
     for (int k = 0; k < 30; k++) {
       const bool odd = (xa & 1u) != 0;
       const bool swap = odd && xa < xb;

@@ -102,6 +102,9 @@ struct MsmConfig {
   uint32_t* bucket_out = nullptr;
   const uint32_t* bucket_add = nullptr;
   cudaEvent_t bucket_ready = nullptr;
+  // The sum in XYZZ coordinates goes here and the affine conversion (an inversion, 31 us of one
+  // thread) is left to the caller: d_out is then not written.  Not with bucket_out or n = 0.
+  uint32_t* xyzz_out = nullptr;
 };
 
 // Bytes of device scratch one MSM of n terms needs (G2 when ec2).

@@ -46,7 +46,8 @@ __global__ void k_bcount(const BatchJob* __restrict__ jobs, uint32_t njobs, uint
   if (!load_scalar<F>(jb.scalars, jb.points, i, k)) return;
   const uint32_t B = 1u << (jb.c - 1);
   for_each_digit(k, (int)jb.c, (int)jb.W, [&](int j, uint32_t mag, bool) {
-    atomicAdd(&counts[jb.bucket0 + (jb.fixed ? 0 : (size_t)j * B) + (mag - 1)], 1u);
+    const size_t b = jb.bucket0 + (jb.fixed ? 0 : (size_t)j * B) + (mag - 1);
+    if (j == 0) claim_shared(counts, b); else atomicAdd(&counts[b], 1u);
   });
 }
 
@@ -60,10 +61,9 @@ __global__ void k_bscatter(const BatchJob* __restrict__ jobs, uint32_t njobs, ui
   uint32_t k[8];
   if (!load_scalar<F>(jb.scalars, jb.points, i, k)) return;
   const uint32_t B = 1u << (jb.c - 1);
-  for_each_digit(k, (int)jb.c, (int)jb.W, [&](int j, uint32_t mag, bool neg) {
-    const uint32_t pos = atomicAdd(&cursor[jb.bucket0 + (jb.fixed ? 0 : (size_t)j * B) + (mag - 1)], 1u);
-    entries[pos] = (jb.fixed ? (uint32_t)j * jb.n + i : i) | (neg ? NEG_BIT : 0u);
-  });
+  scatter_digits(k, (int)jb.c, (int)jb.W, cursor, entries,
+                 [&](int j, uint32_t mag) { return jb.bucket0 + (jb.fixed ? 0 : (size_t)j * B) + (mag - 1); },
+                 [&](int j, bool neg) { return (jb.fixed ? (uint32_t)j * jb.n + i : i) | (neg ? NEG_BIT : 0u); });
 }
 
 // One warp per instance (block i: instance i):
@@ -71,7 +71,7 @@ __global__ void k_bscatter(const BatchJob* __restrict__ jobs, uint32_t njobs, ui
 template <class F>
 __global__ void __launch_bounds__(32) k_bfinish(const BatchJob* __restrict__ jobs, const uint32_t* __restrict__ wsum) {
   const BatchJob jb = jobs[blockIdx.x];
-  windows_horner<F>(wsum + (size_t)jb.window0 * 4 * FieldWords<F>::value, (int)jb.sets, (int)jb.c, jb.out);
+  windows_horner<F>(wsum + (size_t)jb.window0 * 4 * FieldWords<F>::value, (int)jb.sets, (int)jb.c, jb.out, nullptr);
 }
 
 struct BatchLayout {
@@ -153,10 +153,7 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   else
     k_accumulate<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets,
                                                              partials, b.d_jobs);
-  if (latency_mode)
-    k_combine_group<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
-  else
-    k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, nb, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(3);
   const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;

@@ -102,6 +102,20 @@ CSB_DEV bool load_scalar(const uint32_t* scalars, const uint32_t* points, uint32
   return !point_is_inf<F>(points + (size_t)i * PW);
 }
 
+// Claims a place in bucket b: its old count or cursor plus this lane's rank among the converged
+// lanes that claim in the same bucket, with one atomic for all of them.  Used for the lowest
+// window only: a witness's bits and small values crowd into a few of its buckets, where atomics
+// to one address run one after another (100,003 terms, half of them 0 or 1: see k_count).
+CSB_DEV uint32_t claim_shared(uint32_t* slots, size_t b) {
+  const uint32_t act = __activemask(), lane = threadIdx.x & 31;
+  const uint32_t peers = __match_any_sync(act, (unsigned long long)b);
+  uint32_t base = 0;
+  const int leader = __ffs((int)peers) - 1;
+  if ((int)lane == leader) base = atomicAdd(&slots[b], (uint32_t)__popc(peers));
+  base = __shfl_sync(peers, base, leader);
+  return base + __popc(peers & ((1u << lane) - 1u));
+}
+
 // Entry placement.  Generic: bucket (window j, |d|-1) of W*B, entry = point index i.
 // Fixed-base (tables T[j*n + i] = 2^(c j) P_i): one set of B buckets, bucket |d|-1,
 // entry = table index j*n + i, so no per-window sums and no Horner step remain.
@@ -114,8 +128,37 @@ __global__ void k_count(const uint32_t* __restrict__ scalars, const uint32_t* __
   if (!load_scalar<F>(scalars, points, i, k)) return;
   const uint32_t B = 1u << (c - 1);
   for_each_digit(k, c, W, [&](int j, uint32_t mag, bool) {
-    atomicAdd(&counts[(FIXED ? 0 : (size_t)j * B) + (mag - 1)], 1u);
+    const size_t b = (FIXED ? 0 : (size_t)j * B) + (mag - 1);
+    if (j == 0) claim_shared(counts, b); else atomicAdd(&counts[b], 1u);
   });
+}
+
+// Writes entry(j, negative) of every nonzero digit into a place of bucket(j, |d|), four
+// windows' atomics in flight at a time: one after another they cost about 1 us each (21 us for
+// the 20 windows of 4096 terms).
+template <class BucketFn, class EntryFn>
+CSB_DEV void scatter_digits(const uint32_t (&k)[8], int c, int W, uint32_t* cursor, uint32_t* entries, BucketFn bucket,
+                            EntryFn entry) {
+  const uint32_t half = 1u << (c - 1), full = 1u << c;
+  uint32_t carry = 0;
+#pragma unroll 1
+  for (int j0 = 0; j0 < W; j0 += 4) {
+    uint32_t mag[4], neg[4], pos[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint32_t raw = j0 + q < W ? scalar_bits(k, (j0 + q) * c, c) + carry : 0u;
+      neg[q] = raw > half;
+      carry = neg[q];
+      mag[q] = neg[q] ? full - raw : raw;
+    }
+    if (j0 == 0 && mag[0]) pos[0] = claim_shared(cursor, bucket(0, mag[0]));
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (mag[q] && j0 + q > 0) pos[q] = atomicAdd(&cursor[bucket(j0 + q, mag[q])], 1u);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (mag[q]) entries[pos[q]] = entry(j0 + q, neg[q] != 0);
+  }
 }
 
 template <class F, bool FIXED>
@@ -127,10 +170,9 @@ __global__ void k_scatter(const uint32_t* __restrict__ scalars, const uint32_t* 
   uint32_t k[8];
   if (!load_scalar<F>(scalars, points, i, k)) return;
   const uint32_t B = 1u << (c - 1);
-  for_each_digit(k, c, W, [&](int j, uint32_t mag, bool neg) {
-    const uint32_t pos = atomicAdd(&cursor[(FIXED ? 0 : (size_t)j * B) + (mag - 1)], 1u);
-    entries[pos] = (FIXED ? (uint32_t)j * n + i : i) | (neg ? NEG_BIT : 0u);
-  });
+  scatter_digits(k, c, W, cursor, entries,
+                 [&](int j, uint32_t mag) { return (FIXED ? 0 : (size_t)j * B) + (mag - 1); },
+                 [&](int j, bool neg) { return (FIXED ? (uint32_t)j * n + i : i) | (neg ? NEG_BIT : 0u); });
 }
 
 // GLV split of a generic G1 MSM: k_i P_i = k1 P_i + k2 phi(P_i) with k_i = k1 + k2 lambda
@@ -185,7 +227,10 @@ __global__ void k_count_glv(const uint32_t* __restrict__ s2, uint32_t n, int c, 
   uint32_t t[8];
   ld_limbs8(t, s2 + (size_t)i * 8);
   const uint32_t B = 1u << (c - 1);
-  for_each_glv_digit(t, c, W, [&](int, int j, uint32_t mag, bool) { atomicAdd(&counts[(size_t)j * B + (mag - 1)], 1u); });
+  for_each_glv_digit(t, c, W, [&](int, int j, uint32_t mag, bool) {
+    const size_t b = (size_t)j * B + (mag - 1);
+    if (j == 0) claim_shared(counts, b); else atomicAdd(&counts[b], 1u);
+  });
 }
 
 template <class F>
@@ -196,10 +241,13 @@ __global__ void k_scatter_glv(const uint32_t* __restrict__ s2, uint32_t n, int c
   uint32_t t[8];
   ld_limbs8(t, s2 + (size_t)i * 8);
   const uint32_t B = 1u << (c - 1);
-  for_each_glv_digit(t, c, W, [&](int h, int j, uint32_t mag, bool neg) {
-    const uint32_t pos = atomicAdd(&cursor[(size_t)j * B + (mag - 1)], 1u);
-    entries[pos] = i | (h ? PHI_BIT : 0u) | (neg ? NEG_BIT : 0u);
-  });
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const uint32_t k[8] = {t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3] & 0x7fffffffu, 0u, 0u, 0u, 0u};
+    const bool sgn = (t[4 * h + 3] >> 31) != 0;
+    scatter_digits(k, c, W, cursor, entries, [&](int j, uint32_t mag) { return (size_t)j * B + (mag - 1); },
+                   [&](int, bool neg) { return i | (h ? PHI_BIT : 0u) | (neg != sgn ? NEG_BIT : 0u); });
+  }
 }
 
 // The base of an entry: P_i, or phi(P_i) = (phix[i], y_i) for a GLV k2 entry (phix given).
@@ -238,9 +286,14 @@ CSB_DEV uint32_t job_of_bucket(const BatchJob* jobs, uint32_t njobs, uint32_t b)
   }
   return lo;
 }
+// Partial sums to add up: `count` of them from slot pbase on, `stride` slots apart, into dst (as a
+// task's).  A bucket of up to kCombineSerial partial sums is one such sum; one of more has each
+// run of kCombineSerial summed into the run's first slot and then, in a second pass, those
+// (stride kCombineSerial), so no thread adds up more than a few of a crowded bucket's thousands.
 struct Multi {
-  uint32_t bucket, pbase, count, pad;
+  uint32_t dst, pbase, count, stride;
 };
+constexpr uint32_t kCombineSerial = 8;
 
 // Task lengths are in [1, TASK]; tasks are emitted in descending length (a counting sort
 // over TASK+1 bins) so the 32 lanes of a warp walk buckets of nearly equal size.
@@ -310,21 +363,47 @@ __global__ void k_task_emit(const uint32_t* __restrict__ offsets, uint32_t nb, u
   __syncthreads();
   for (int i = threadIdx.x; i <= kMaxTask; i += blockDim.x) cnt_s[i] = 0;
   __syncthreads();
-  if (cnt == 0) return;
-  const uint32_t nt = nfull + 1;
-  const uint32_t job = jobs ? job_of_bucket(jobs, njobs, b) : 0u;
-  uint32_t pbase = 0;
+  const uint32_t nt = cnt ? nfull + 1 : 0u;
+  const uint32_t job = jobs && cnt ? job_of_bucket(jobs, njobs, b) : 0u;
+  uint32_t pbase = 0, mslot = 0;
   if (nt > 1) {
     pbase = atomicAdd(&counters[1], nt);
-    const uint32_t mslot = atomicAdd(&counters[2], 1u);
-    multi[mslot] = {b, pbase, nt, 0u};
+    mslot = atomicAdd(&counters[2], nt > kCombineSerial ? 1 + (nt + kCombineSerial - 1) / kCombineSerial : 1u);
+    multi[mslot] = nt > kCombineSerial ? Multi{b, pbase, (nt + kCombineSerial - 1) / kCombineSerial, kCombineSerial}
+                                       : Multi{b, pbase, nt, 1u};
   }
+  // a crowded bucket's records are written by the whole warp
+  constexpr uint32_t kAlone = 16;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t big = __ballot_sync(0xffffffffu, nt > kAlone); big; big &= big - 1) {
+    const int src = __ffs((int)big) - 1;
+    const uint32_t o_nt = __shfl_sync(0xffffffffu, nt, src), o_start = __shfl_sync(0xffffffffu, start, src);
+    const uint32_t o_last = __shfl_sync(0xffffffffu, last, src), o_pbase = __shfl_sync(0xffffffffu, pbase, src);
+    const uint32_t o_mslot = __shfl_sync(0xffffffffu, mslot, src), o_job = __shfl_sync(0xffffffffu, job, src);
+    uint32_t at = 0;
+    if ((int)lane == src) at = base_s[task_len] + atomicAdd(&cnt_s[task_len], o_nt - 1);
+    at = __shfl_sync(0xffffffffu, at, src);
+    for (uint32_t t = lane; t < o_nt - 1; t += 32)
+      tasks[at + t] = {o_start + t * task_len, task_len, nb + o_pbase + t, o_job};
+    if ((int)lane == src) {
+      const uint32_t slot = base_s[o_last] + atomicAdd(&cnt_s[o_last], 1u);
+      tasks[slot] = {o_start + (o_nt - 1) * task_len, o_last, nb + o_pbase + o_nt - 1, o_job};
+    }
+    for (uint32_t q = lane; q * kCombineSerial < o_nt; q += 32)
+      multi[o_mslot + 1 + q] = {nb + o_pbase + q * kCombineSerial, o_pbase + q * kCombineSerial,
+                                min(kCombineSerial, o_nt - q * kCombineSerial), 1u};
+  }
+  if (nt == 0 || nt > kAlone) return;
 #pragma unroll 1
   for (uint32_t t = 0; t < nt; t++) {
     const uint32_t len = t < nfull ? task_len : last;
     const uint32_t slot = base_s[len] + atomicAdd(&cnt_s[len], 1u);
     tasks[slot] = {start + t * task_len, len, nt == 1 ? b : nb + pbase + t, job};
   }
+  if (nt > kCombineSerial)
+    for (uint32_t q = 0; q * kCombineSerial < nt; q++)
+      multi[mslot + 1 + q] = {nb + pbase + q * kCombineSerial, pbase + q * kCombineSerial,
+                              min(kCombineSerial, nt - q * kCombineSerial), 1u};
 }
 
 // Minimum resident blocks per SM asked of the compiler for the accumulation kernel: G1 at 4
@@ -443,34 +522,14 @@ __global__ void __launch_bounds__(128) k_add_buckets(uint32_t* __restrict__ buck
   st_xyzz<F>(buckets + (size_t)b * XW, xyzz_add(x, y));
 }
 
-// Split buckets with at most kCombineSerial partials: one thread each, a serial sum.
-// (The top window of a scalar has fewer bits, so its digits crowd into fewer buckets and
-// many of those split into two or three tasks.)
-constexpr uint32_t kCombineSerial = 8;
-
+// First pass: one group of lanes per sum of at most kCombineSerial neighbouring partial sums
+// (few of them, and a chain each: one thread per sum took 131 us over Fq2 where a group takes
+// 20).  The top window of a scalar has fewer bits, so its digits crowd into fewer buckets and
+// many of those split.
 template <class F>
-__global__ void __launch_bounds__(128) k_combine_small(const Multi* __restrict__ multi,
-                                                       const uint32_t* __restrict__ counters,
-                                                       const uint32_t* __restrict__ partials,
-                                                       uint32_t* __restrict__ buckets) {
-  constexpr int XW = 4 * FieldWords<F>::value;
-  const uint32_t nm = counters[2];
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < nm; m += gridDim.x * blockDim.x) {
-    const Multi mu = multi[m];
-    if (mu.count > kCombineSerial) continue;
-    XYZZ<F> acc = ld_xyzz<F>(partials + (size_t)mu.pbase * XW);
-#pragma unroll 1
-    for (uint32_t i = 1; i < mu.count; i++) acc = xyzz_add(acc, ld_xyzz<F>(partials + (size_t)(mu.pbase + i) * XW));
-    st_xyzz<F>(buckets + (size_t)mu.bucket * XW, acc);
-  }
-}
-
-// k_combine_small with one group of lanes per split bucket (the latency form's).
-template <class F>
-__global__ void __launch_bounds__(128, 4) k_combine_group(const Multi* __restrict__ multi,
-                                                       const uint32_t* __restrict__ counters,
-                                                       const uint32_t* __restrict__ partials,
-                                                       uint32_t* __restrict__ buckets) {
+__global__ void __launch_bounds__(128, 4) k_combine_small(const Multi* __restrict__ multi,
+                                                          const uint32_t* __restrict__ counters, uint32_t nb,
+                                                          uint32_t* partials, uint32_t* __restrict__ buckets) {
   using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
   constexpr uint32_t G = Gr::G, GPW = 32 / G, NG = 128 / G;
@@ -483,7 +542,7 @@ __global__ void __launch_bounds__(128, 4) k_combine_group(const Multi* __restric
   for (uint32_t first = warp0 * GPW; first < nm; first += nwarps * GPW) {  // warp-uniform
     const uint32_t m = first + (threadIdx.x & 31) / G;
     Multi mu = m < nm ? multi[m] : Multi{0, 0, 0, 0};
-    if (mu.count > kCombineSerial) mu.count = 0;  // k_combine
+    if (mu.stride != 1) mu.count = 0;  // k_combine
     const uint32_t steps = __reduce_max_sync(0xffffffffu, mu.count);
     grp.load(acc, partials + (size_t)mu.pbase * XW, mu.count != 0);
 #pragma unroll 1
@@ -491,54 +550,41 @@ __global__ void __launch_bounds__(128, 4) k_combine_group(const Multi* __restric
       const bool live = i < mu.count;
       grp.add(acc, acc, live ? partials + (size_t)(mu.pbase + i) * XW : acc, live);
     }
-    if (mu.count) grp.store(buckets + (size_t)mu.bucket * XW, acc);
+    if (mu.count)
+      grp.store(mu.dst < nb ? buckets + (size_t)mu.dst * XW : partials + (size_t)(mu.dst - nb) * XW, acc);
     __syncwarp();
   }
 }
 
-// Split buckets with more partials: one block each, tree sum.
+// Second pass: the runs of a bucket with more partial sums, one block each: every group adds up
+// its share, then a tree over the groups.
 template <class F>
-__global__ void __launch_bounds__(128) k_combine(const Multi* __restrict__ multi,
-                                                 const uint32_t* __restrict__ counters,
-                                                 const uint32_t* __restrict__ partials,
-                                                 uint32_t* __restrict__ buckets) {
+__global__ void __launch_bounds__(128, 4) k_combine(const Multi* __restrict__ multi,
+                                                    const uint32_t* __restrict__ counters,
+                                                    const uint32_t* __restrict__ partials,
+                                                    uint32_t* __restrict__ buckets) {
+  using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
-  __shared__ uint32_t red[4][XW];
+  constexpr uint32_t G = Gr::G, NG = 128 / G;
+  __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const uint32_t g = threadIdx.x / G;
+  const Gr grp(scr[g]);
+  uint32_t* acc = accs[g];
   const uint32_t nm = counters[2];
   for (uint32_t m = blockIdx.x; m < nm; m += gridDim.x) {
     const Multi mu = multi[m];
-    if (mu.count <= kCombineSerial) continue;  // k_combine_small
-    XYZZ<F> acc = XYZZ<F>::inf();
+    if (mu.stride == 1) continue;  // first pass (the whole block leaves together)
+    auto at = [&](uint32_t i) { return partials + (size_t)(mu.pbase + i * mu.stride) * XW; };
+    grp.load(acc, at(g), g < mu.count);
 #pragma unroll 1
-    for (uint32_t i = threadIdx.x; i < mu.count; i += blockDim.x)
-      acc = xyzz_add_cold(acc, ld_xyzz<F>(partials + (size_t)(mu.pbase + i) * XW));
-    // warp tree
-#pragma unroll 1
-    for (int d = 16; d > 0; d >>= 1) {
-      XYZZ<F> o;
-      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-      const uint32_t* aw = reinterpret_cast<const uint32_t*>(&acc);
-#pragma unroll
-      for (int w = 0; w < XW; w++) ow[w] = __shfl_down_sync(0xffffffffu, aw[w], d);
-      acc = xyzz_add_cold(acc, o);
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-      const uint32_t* aw = reinterpret_cast<const uint32_t*>(&acc);
-      for (int w = 0; w < XW; w++) red[warp][w] = aw[w];
-    }
+    for (uint32_t i = NG; i < mu.count; i += NG) grp.add(acc, acc, i + g < mu.count ? at(i + g) : acc, i + g < mu.count);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      XYZZ<F> s = XYZZ<F>::inf();
 #pragma unroll 1
-      for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-        XYZZ<F> o;
-        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-        for (int w = 0; w < XW; w++) ow[w] = red[k][w];
-        s = xyzz_add_cold(s, o);
-      }
-      st_xyzz<F>(buckets + (size_t)mu.bucket * XW, s);
+    for (uint32_t d = NG / 2; d >= 1; d >>= 1) {
+      grp.add(acc, acc, accs[(g + d) & (NG - 1)], g < d);
+      __syncthreads();
     }
+    if (g == 0) grp.store(buckets + (size_t)mu.dst * XW, acc);
     __syncthreads();
   }
 }
@@ -662,12 +708,10 @@ __global__ void __launch_bounds__(32) k_window_horner(const uint32_t* __restrict
     grp.dbl(acc, acc);
     grp.add(acc, acc, has(i) ? T(i) : acc, has(i));
   }
-#pragma unroll 1
-  for (int i = 0; i < s; i++) grp.dbl(acc, acc, upper);
   uint32_t* a0 = accs[0];
+  double_times<F>(grp, acc, s, upper);
   grp.add(acc, acc, accs[(threadIdx.x / G) | 1], !upper);
-#pragma unroll 1
-  for (int i = 0; i < shift; i++) grp.dbl(acc, acc);
+  double_times<F>(grp, acc, shift);
   grp.add(acc, acc, yw, !upper);
   if (z) grp.add(acc, acc, z + (size_t)blockIdx.x * n * XW, !upper);
   if (threadIdx.x >= G) return;
@@ -680,7 +724,7 @@ __global__ void __launch_bounds__(32) k_window_horner(const uint32_t* __restrict
 
 // sum_j 2^(c j) S_j (Horner over the windows) and the affine result.
 template <class F>
-CSB_DEV void windows_horner(const uint32_t* wsum, int W, int c, uint32_t* out) {
+CSB_DEV void windows_horner(const uint32_t* wsum, int W, int c, uint32_t* out, uint32_t* xyzz_out) {
   // one warp; its groups compute the same
   using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
@@ -691,16 +735,19 @@ CSB_DEV void windows_horner(const uint32_t* wsum, int W, int c, uint32_t* out) {
   grp.load(acc, wsum + (size_t)(W - 1) * XW);
 #pragma unroll 1
   for (int j = W - 2; j >= 0; j--) {
-#pragma unroll 1
-    for (int d = 0; d < c; d++) grp.dbl(acc, acc);
+    double_times<F>(grp, acc, c);
     grp.add(acc, acc, wsum + (size_t)j * XW);
   }
-  if ((threadIdx.x & 31) == 0) Gr::store_affine(out, acc);
+  if (xyzz_out) {
+    if ((threadIdx.x & 31) < G) grp.store(xyzz_out, acc);
+  } else if ((threadIdx.x & 31) == 0) {
+    Gr::store_affine(out, acc);
+  }
 }
 template <class F>
 __global__ void __launch_bounds__(32) k_finish(const uint32_t* __restrict__ wsum, int W, int c,
-                                               uint32_t* __restrict__ out) {
-  windows_horner<F>(wsum, W, c, out);
+                                               uint32_t* __restrict__ out, uint32_t* __restrict__ xyzz_out) {
+  windows_horner<F>(wsum, W, c, out, xyzz_out);
 }
 
 template <class F>
@@ -874,7 +921,7 @@ static_assert(kCtrHist + kMaxTask + 1 <= kCtrCursor && kCtrCursor + kMaxTask + 1
               "task-length bins must not overlap");
 // the reduction runs eight buckets per thread while the remaining values times a group's lanes
 // exceed this many times the resident threads
-constexpr uint64_t kTreeFill = 4;
+constexpr uint64_t kTreeFill = 16;
 
 struct Layout {
   size_t counts, offsets, entries, tasks, multi, partials, buckets, lv_y, lv_z, lv_y2, lv_z2, wsum,
@@ -1021,6 +1068,7 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
                      cudaStream_t st) {
   constexpr bool EC2 = FieldWords<F>::value == 16;
   constexpr int XB = 4 * FieldWords<F>::value * 4;  // bytes per XYZZ point
+  if (cfg.xyzz_out && n_in == 0) return cudaErrorInvalidValue;
   // shared buckets: fixed-base MSMs (one bucket set) with terms (the accumulation is what
   // writes every bucket of the array)
   if ((cfg.bucket_out || cfg.bucket_add) && (!FIXED || n_in == 0)) return cudaErrorInvalidValue;
@@ -1158,10 +1206,7 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
     k_accumulate<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, acc_entries, acc_points, nb,
                                                              buckets, partials, nullptr, phix);
   note_launch();
-  if (latency_mode)
-    k_combine_group<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
-  else
-    k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
+  k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, nb, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(2);
   if (cfg.acc_stop) cudaEventRecord(cfg.acc_stop, st);
@@ -1177,9 +1222,10 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
     k_add_buckets<F><<<(B + 127) / 128, 128, 0, st>>>(buckets, cfg.bucket_add, B);
     note_launch();
   }
-  reduce_buckets<F>(buckets, B, (uint32_t)WR, lv_y, lv_z, lv_y2, lv_z2, wsum, WR == 1 ? d_out : nullptr, resident, st);
+  reduce_buckets<F>(buckets, B, (uint32_t)WR, lv_y, lv_z, lv_y2, lv_z2, cfg.xyzz_out && WR == 1 ? cfg.xyzz_out : wsum,
+                    WR == 1 && !cfg.xyzz_out ? d_out : nullptr, resident, st);
   if (WR > 1) {
-    k_finish<F><<<1, 32, 0, st>>>(wsum, WR, c, d_out);
+    k_finish<F><<<1, 32, 0, st>>>(wsum, WR, c, d_out, cfg.xyzz_out);
     note_launch();
   }
   return cudaGetLastError();
