@@ -146,27 +146,35 @@ inline GlvSplit split(const uint32_t* k32) {
 }
 }  // namespace glv_host
 
-// out (XYZZ) = k * P for P affine (G1), k given as its GLV split: k P = k1 P + phi(k2 P).
+// out (XYZZ) = k * P (G1), k given as its GLV split: k P = k1 P + phi(k2 P).  P is affine, or
+// XYZZ where xyzz_in; its affine form then goes to affine_out if that is given, from another warp
+// meanwhile.
 // One block of 128 threads, 32 groups of lanes (group.cuh).  The 127 doublings 2^i P are one
 // chain (its first warp); the sums over the set bits of k1 and k2 are not: 16 groups each add
-// up 8 of the 2^i P, a tree joins them, and phi and the signs come last: 435 dependent
-// products instead of the 760 of a joint double-and-add.
+// up 8 of the 2^i P, a tree joins them, and phi and the signs come last: 310 dependent
+// products instead of the 760 of a joint double-and-add (187 us against 450).
 constexpr int kScaleThreads = 128;
-__device__ void scale_point_glv(const uint32_t* __restrict__ P, const GlvSplit* __restrict__ gs,
-                                uint32_t* __restrict__ out) {
+__device__ void scale_point_glv(const uint32_t* __restrict__ P, bool xyzz_in, const GlvSplit* __restrict__ gs,
+                                uint32_t* __restrict__ out, uint32_t* __restrict__ affine_out) {
   using Gr = Group<Fq>;
   __shared__ __align__(16) uint32_t scr[32][Gr::kScratch], pw[128][32], acc[32][32];
   const uint32_t g = threadIdx.x / Gr::G;
   const Gr grp(scr[g]);
-  if (threadIdx.x < 32) {  // 2^i P (every group of the warp computes and stores the same)
-    const Affine<Fq> p = ld_affine<Fq>(P);
-    const XYZZ<Fq> x = affine_is_inf(p) ? XYZZ<Fq>::inf() : XYZZ<Fq>::from_affine(p);
+  if (threadIdx.x < 32) {  // 2^i P (every group of the warp computes the same, the first one stores)
     if (threadIdx.x == 0) {
+      XYZZ<Fq> x = XYZZ<Fq>::inf();
+      if (xyzz_in) {
+        x = ld_xyzz<Fq>(P);
+      } else {
+        const Affine<Fq> p = ld_affine<Fq>(P);
+        if (!affine_is_inf(p)) x = XYZZ<Fq>::from_affine(p);
+      }
       sts_fq(pw[0], x.X); sts_fq(pw[0] + 8, x.Y); sts_fq(pw[0] + 16, x.ZZ); sts_fq(pw[0] + 24, x.ZZZ);
     }
     __syncwarp();
-#pragma unroll 1
-    for (int i = 1; i < 128; i++) grp.dbl(pw[i], pw[i - 1], g == 0);
+    doubling_run(scr[g], pw[0], 127, pw[0], g == 0);
+  } else if (threadIdx.x == 32 && affine_out) {
+    st_affine<Fq>(affine_out, xyzz_to_affine(ld_xyzz<Fq>(P)));
   }
   __syncthreads();
   const uint32_t half = g >> 4, b0 = 8 * (g & 15);
@@ -196,13 +204,14 @@ __device__ void scale_point_glv(const uint32_t* __restrict__ P, const GlvSplit* 
 }
 __global__ void __launch_bounds__(kScaleThreads) k_scale_point_glv(const uint32_t* __restrict__ P,
                                                                    const GlvSplit* __restrict__ gs,
-                                                                   uint32_t* __restrict__ out) {
-  scale_point_glv(P, gs, out);
+                                                                   uint32_t* __restrict__ out,
+                                                                   uint32_t* __restrict__ affine_out) {
+  scale_point_glv(P, true, gs, out, affine_out);
 }
 
-// pi_C = C2 + C + sA + rB1 (C2, C affine; sA, rB1 XYZZ) -> affine; one warp (its first group of
-// lanes; the others compute on copies)
-__device__ void final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c,
+// pi_C = C2 + C + sA + rB1 -> affine (sA, rB1 XYZZ; C2 and C XYZZ, or affine where affine_in; C may
+// be null); one warp (its first group of lanes; the others compute on copies)
+__device__ void final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c, bool affine_in,
                         const uint32_t* __restrict__ sa, const uint32_t* __restrict__ rb1,
                         uint32_t* __restrict__ out) {
   using Gr = Group<Fq>;
@@ -210,17 +219,21 @@ __device__ void final_c(const uint32_t* __restrict__ c2, const uint32_t* __restr
   const uint32_t g = (threadIdx.x & 31) / Gr::G;
   const Gr grp(scr[g]);
   uint32_t* acc = accs[g];
-  grp.load(acc, nullptr, false);
-  grp.madd(acc, acc, c2, c2 + 8, false, !affine_is_inf(ld_affine<Fq>(c2)));
-  grp.madd(acc, acc, c, c + 8, false, !affine_is_inf(ld_affine<Fq>(c)));
-  grp.add(acc, acc, sa);
+  grp.load(acc, sa);
   grp.add(acc, acc, rb1);
+  if (affine_in) {
+    grp.madd(acc, acc, c2, c2 + 8, false, !affine_is_inf(ld_affine<Fq>(c2)));
+    grp.madd(acc, acc, c, c + 8, false, !affine_is_inf(ld_affine<Fq>(c)));
+  } else {
+    grp.add(acc, acc, c2);
+    if (c) grp.add(acc, acc, c);
+  }
   if ((threadIdx.x & 31) == 0) Gr::store_affine(out, acc);
 }
 __global__ void __launch_bounds__(32) k_final_c(const uint32_t* __restrict__ c2, const uint32_t* __restrict__ c,
                                                 const uint32_t* __restrict__ sa, const uint32_t* __restrict__ rb1,
                                                 uint32_t* __restrict__ out) {
-  final_c(c2, c, sa, rb1, out);
+  final_c(c2, c, false, sa, rb1, out);
 }
 
 cudaError_t copy_in(void* dst, const void* src, size_t bytes, int on_device, cudaStream_t st) {
@@ -272,7 +285,7 @@ ProvePlan plan_prove(const cs_pk* pk) {
   P.ms_b2 = o; o += al256(P.bytes_b2);
   P.ms_c = o; o += al256(P.bytes_c);
   P.ms_h = o; o += al256(P.bytes_h);
-  P.pts = o; o += 2048;   // outA 64, outB1 64, outB2 128, outC 64, outH 64, sA 128, rB1 128, piC 64
+  P.pts = o; o += 2048;   // outA 64, outB1 64, outB2 128, outC 64, outH 64, sA, rB1 128, piC 64, xA, xB1, xC, xH 128
   P.rs = o; o += 256;     // r, s, -rs, then the GLV splits of s and r (2 x 64 B)
   P.share_ch = pk->has_fixed() && pk->fc.c > 0 && pk->fc.c == pk->fh.c && pk->fc.n > 0 && pk->fh.n > 0;
   P.cbk = o;
@@ -281,27 +294,25 @@ ProvePlan plan_prove(const cs_pk* pk) {
   return P;
 }
 
-// The proof's launch sequence after the scalar uploads (which cs_prove_device makes): the
-// witness scalars with their extensions, the four witness MSMs on the auxiliary streams with
-// the GLV scalings, QAP -> H step -> H MSM on the H stream, the join and the final pi_C.
-// Results land in the scratch's point area.  Sets *where on failure.
-cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_t* d_w, Domain* dom1,
-                       Domain* dom2, const char** where) {
+// The proof's launch sequence after the uploads (which cs_prove_device makes: r, s and the
+// witness, copied to wA): the witness scalars' extensions, the four witness MSMs on the
+// auxiliary streams with the GLV scalings, QAP -> H step -> H MSM on the H stream, the join and
+// the final pi_C.  Results land in the scratch's point area.  Sets *where on failure.
+cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1, Domain* dom2, const char** where) {
   char* base = static_cast<char*>(ctx->work.ptr);
   auto at = [&](size_t off) { return reinterpret_cast<uint32_t*>(base + off); };
   uint32_t *wA = at(P.wA), *wB = at(P.wB), *pA = at(P.pA), *pB = at(P.pB), *M = at(P.M), *hscr = at(P.hscr);
   uint32_t* pts = at(P.pts);
   uint32_t *outA = pts, *outB1 = pts + 16, *outB2 = pts + 32, *outC = pts + 64, *outH = pts + 80;
   uint32_t *sA = pts + 96, *rB1 = pts + 128, *piC = pts + 160;
+  uint32_t *xA = pts + 176, *xB1 = pts + 208, *xC = pts + 240, *xH = pts + 272;  // XYZZ
   uint32_t* rs = at(P.rs);
   const uint32_t nv = pk->n_vars, m = pk->m, np1 = pk->n_public + 1;
   cudaStream_t s0 = ctx->stream;
   cudaEvent_t ev_w = ctx->aux_ev[0];
-  MsmConfig cfg;
   cudaError_t e;
   // scalars: w ++ [1, r] and w ++ [1, s]; -rs
-  bool ok = (e = cudaMemcpyAsync(wA, d_w, (size_t)nv * 32, cudaMemcpyDeviceToDevice, s0)) == cudaSuccess &&
-            (e = cudaMemcpyAsync(wB, d_w, (size_t)nv * 32, cudaMemcpyDeviceToDevice, s0)) == cudaSuccess;
+  bool ok = (e = cudaMemcpyAsync(wB, wA, (size_t)nv * 32, cudaMemcpyDeviceToDevice, s0)) == cudaSuccess;
   if (!ok) { *where = "prove inputs"; return e; }
   k_set_tail<<<1, 32, 0, s0>>>(wA, nv, rs);
   k_set_tail<<<1, 32, 0, s0>>>(wB, nv, rs + 8);
@@ -314,23 +325,28 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
   // resident fixed-base tables when the key has them, else the generic MSM over the points
   auto run_msm = [&](bool ec2, const uint32_t* sc, const uint32_t* pts, const cs_pk::Fixed& f, uint32_t n,
                      uint32_t* out, size_t off, size_t bytes, cudaStream_t st, const MsmConfig* share = nullptr) {
+    MsmConfig fcfg = share ? *share : MsmConfig{};
     if (pk->has_fixed()) {
-      MsmConfig fcfg = share ? *share : MsmConfig{};
       fcfg.c = f.c;
       return ec2 ? msm_fixed_g2(sc, f.table, n, out, at(off), bytes, fcfg, st)
                  : msm_fixed_g1(sc, f.table, n, out, at(off), bytes, fcfg, st);
     }
-    return ec2 ? msm_g2(sc, pts, n, out, at(off), bytes, cfg, st) : msm_g1(sc, pts, n, out, at(off), bytes, cfg, st);
+    return ec2 ? msm_g2(sc, pts, n, out, at(off), bytes, fcfg, st) : msm_g1(sc, pts, n, out, at(off), bytes, fcfg, st);
   };
-  // C hands its buckets to H (outC is then the point at infinity, and outH the sum of both)
-  MsmConfig share_c, share_h;
+  // The G1 sums stay in XYZZ coordinates: only pi_A (beside its scaling) and pi_C are converted.
+  // C hands its buckets to H (xH is then the sum of both)
+  MsmConfig cfg_a, cfg_b1, share_c, share_h;
+  cfg_a.xyzz_out = xA;
+  cfg_b1.xyzz_out = xB1;
+  share_h.xyzz_out = xH;
+  if (!P.share_ch) share_c.xyzz_out = xC;
   if (P.share_ch) {
     share_c.bucket_out = at(P.cbk);
     share_h.bucket_add = at(P.cbk);
     share_h.bucket_ready = ctx->aux_ev[7];
   }
-  ok = (e = run_msm(false, wA, pk->a_ext, pk->fa, nv + 2, outA, P.ms_a, P.bytes_a, sa)) == cudaSuccess &&
-       (e = run_msm(false, wB, pk->b1_ext, pk->fb1, nv + 2, outB1, P.ms_b1, P.bytes_b1, sb1)) == cudaSuccess &&
+  ok = (e = run_msm(false, wA, pk->a_ext, pk->fa, nv + 2, outA, P.ms_a, P.bytes_a, sa, &cfg_a)) == cudaSuccess &&
+       (e = run_msm(false, wB, pk->b1_ext, pk->fb1, nv + 2, outB1, P.ms_b1, P.bytes_b1, sb1, &cfg_b1)) == cudaSuccess &&
        (e = run_msm(true, wB, pk->b2_ext, pk->fb2, nv + 2, outB2, P.ms_b2, P.bytes_b2, sb2)) == cudaSuccess &&
        (e = run_msm(false, wA + (size_t)np1 * 8, pk->c + (size_t)np1 * 16, pk->fc, nv - np1, outC, P.ms_c, P.bytes_c,
                     sc, &share_c)) == cudaSuccess;
@@ -338,15 +354,15 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
   if (P.share_ch && (e = cudaEventRecord(ctx->aux_ev[7], sc)) != cudaSuccess) { *where = "prove C buckets"; return e; }
   {
     const GlvSplit* gsp = reinterpret_cast<const GlvSplit*>(rs + 32);
-    k_scale_point_glv<<<1, kScaleThreads, 0, sa>>>(outA, gsp, sA);        // s * pi_A
-    k_scale_point_glv<<<1, kScaleThreads, 0, sb1>>>(outB1, gsp + 1, rB1);  // r * pi_B1
+    k_scale_point_glv<<<1, kScaleThreads, 0, sa>>>(xA, gsp, sA, outA);             // s * pi_A
+    k_scale_point_glv<<<1, kScaleThreads, 0, sb1>>>(xB1, gsp + 1, rB1, nullptr);  // r * pi_B1
   }
   note_launch(2);
   // QAP evaluation, H step and H MSM on their own stream
   cudaStream_t sh = ctx->aux_h;
   cudaStreamWaitEvent(sh, ev_w, 0);
-  ok = (e = qap_eval(pk->rows_a, d_w, pA, 0, sh)) == cudaSuccess &&
-       (e = qap_eval(pk->rows_b, d_w, pB, 0, sh)) == cudaSuccess &&
+  ok = (e = qap_eval(pk->rows_a, wA, pA, 0, sh)) == cudaSuccess &&
+       (e = qap_eval(pk->rows_b, wA, pB, 0, sh)) == cudaSuccess &&
        (e = hstep_reference_core(pA, pB, pk->log_m, domain_wf(dom2), domain_wi(dom2), domain_wf(dom2),
                                  domain_consts(dom1) + 72, domain_consts(dom2) + 24, M, hscr, sh)) == cudaSuccess &&
        (e = cudaEventRecord(ctx->aux_ev[6], sh)) == cudaSuccess &&  // H step done (stage times)
@@ -362,7 +378,7 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
     cudaEventRecord(ctx->aux_ev[1 + i], ctx->aux[i]);
     cudaStreamWaitEvent(sh, ctx->aux_ev[1 + i], 0);
   }
-  k_final_c<<<1, 32, 0, sh>>>(outH, outC, sA, rB1, piC);
+  k_final_c<<<1, 32, 0, sh>>>(xH, P.share_ch ? nullptr : xC, sA, rB1, piC);
   note_launch();
   cudaEventRecord(ctx->aux_ev[3], ctx->aux[2]);  // B2 done
   cudaEventRecord(ctx->aux_ev[8], sh);           // pi_C done
@@ -371,12 +387,12 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_
   return cudaGetLastError();
 }
 
-// Captures prove_body on the context stream as a CUDA graph, keeps it for the key, witness
-// buffer and scratch, and launches it.  Capture is thread-local, so other threads
+// Captures prove_body on the context stream as a CUDA graph, keeps it for the key and scratch,
+// and launches it.  Capture is thread-local, so other threads
 // (other server slots) keep launching meanwhile.  If the capture or its instantiation fails, the
 // entry records that and the sequence runs launch by launch, now and on later calls.
-cudaError_t prove_capture(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint32_t* d_w, Domain* dom1,
-                          Domain* dom2, const char** where) {
+cudaError_t prove_capture(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1, Domain* dom2,
+                          const char** where) {
   // a served context sees every key of its server: room for that many, the oldest goes first
   // (a graph destroyed while a launch of it runs is freed when the launch completes)
   constexpr size_t kMaxGraphs = 32;
@@ -397,14 +413,13 @@ cudaError_t prove_capture(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint
   }
   cs_ctx::ProveGraph g;
   g.pk_id = pk->id;
-  g.d_w = d_w;
   g.work = ctx->work.ptr;
   g.work_bytes = ctx->work.bytes;
   const unsigned long long l0 = thread_launches();
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    const cudaError_t eb = prove_body(ctx, pk, P, d_w, dom1, dom2, where);
+    const cudaError_t eb = prove_body(ctx, pk, P, dom1, dom2, where);
     e = cudaStreamEndCapture(s0, &graph);
     if (eb != cudaSuccess) e = eb;
   }
@@ -422,7 +437,7 @@ cudaError_t prove_capture(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, const uint
   g.exec = nullptr;
   ctx->prove_graphs.push_back(g);
   *where = "prove launch";
-  return prove_body(ctx, pk, P, d_w, dom1, dom2, where);
+  return prove_body(ctx, pk, P, dom1, dom2, where);
 }
 
 // ------------------------------------------------------------------ proof batches ----
@@ -507,7 +522,7 @@ __global__ void __launch_bounds__(kScaleThreads) k_batch_scale(char* __restrict_
   const uint32_t k = blockIdx.x >> 1, which = blockIdx.x & 1;
   uint32_t* pts = reinterpret_cast<uint32_t*>(base + (size_t)k * per + o_pts);
   const GlvSplit* gs = reinterpret_cast<const GlvSplit*>(base + (size_t)k * per + o_rs + 32 * 4) + which;
-  scale_point_glv(which ? pts + 16 : pts, gs, which ? pts + 128 : pts + 96);
+  scale_point_glv(which ? pts + 16 : pts, false, gs, which ? pts + 128 : pts + 96, nullptr);
 }
 
 // Proof k's H coefficient 2m-1 (always zero) becomes its -r s (block k), the scalar of the
@@ -521,7 +536,7 @@ __global__ void k_batch_rs(char* __restrict__ base, size_t per, size_t o_rs, siz
 // pi_C of every proof (block k): needs the G1 MSMs, their scalings and the H MSMs, not G2.
 __global__ void __launch_bounds__(32) k_batch_pic(char* __restrict__ base, size_t per, size_t o_pts) {
   uint32_t* pts = reinterpret_cast<uint32_t*>(base + (size_t)blockIdx.x * per + o_pts);
-  final_c(pts + 80, pts + 64, pts + 96, pts + 128, pts + 160);
+  final_c(pts + 80, pts + 64, true, pts + 96, pts + 128, pts + 160);
 }
 
 // The proof words of every proof (block k) to the caller's buffer.
@@ -825,11 +840,12 @@ int cs_prove_device(cs_ctx* ctx, cs_pk* pk, const uint32_t* d_w, const uint32_t*
   cudaStream_t s0 = ctx->stream;
   const GlvSplit glv_rs[2] = {glv_host::split(s), glv_host::split(r)};  // s * pi_A, r * pi_B1
   cudaEventRecord(ctx->ev_start, s0);
-  // the call's scalars r, s and their GLV splits go to the device first; everything after
-  // them depends only on the key, the witness buffer and the scratch layout
+  // the call's scalars r, s, their GLV splits and the witness go to the scratch first; everything
+  // after them depends only on the key and the scratch layout
   bool ok = (e = cudaMemcpyAsync(rs, r, 32, cudaMemcpyHostToDevice, s0)) == cudaSuccess &&
             (e = cudaMemcpyAsync(rs + 8, s, 32, cudaMemcpyHostToDevice, s0)) == cudaSuccess &&
-            (e = cudaMemcpyAsync(rs + 32, glv_rs, sizeof(glv_rs), cudaMemcpyHostToDevice, s0)) == cudaSuccess;
+            (e = cudaMemcpyAsync(rs + 32, glv_rs, sizeof(glv_rs), cudaMemcpyHostToDevice, s0)) == cudaSuccess &&
+            (e = cudaMemcpyAsync(base + P.wA, d_w, (size_t)pk->n_vars * 32, cudaMemcpyDeviceToDevice, s0)) == cudaSuccess;
   if (!ok) return fail(ctx, e, "prove inputs");
   const char* where = "prove launch";
   // Graphs pay where launching is a visible part of a proof (small domains: a 2^12 proof
@@ -837,12 +853,12 @@ int cs_prove_device(cs_ctx* ctx, cs_pk* pk, const uint32_t* d_w, const uint32_t*
   // mix of sizes, so those proofs launch directly.
   constexpr uint32_t kGraphMaxDomain = 1u << 17;
   if (!ctx->use_prove_graphs || pk->m > kGraphMaxDomain) {
-    e = prove_body(ctx, pk, P, d_w, dom1, dom2, &where);
+    e = prove_body(ctx, pk, P, dom1, dom2, &where);
     ctx->stages_valid = true;
   } else {
     cs_ctx::ProveGraph* g = nullptr;
     for (auto& x : ctx->prove_graphs)
-      if (x.pk_id == pk->id && x.d_w == d_w && x.work == ctx->work.ptr && x.work_bytes == ctx->work.bytes)
+      if (x.pk_id == pk->id && x.work == ctx->work.ptr && x.work_bytes == ctx->work.bytes)
         g = &x;
     if (g && g->exec) {
       e = cudaGraphLaunch(g->exec, s0);
@@ -850,10 +866,10 @@ int cs_prove_device(cs_ctx* ctx, cs_pk* pk, const uint32_t* d_w, const uint32_t*
       where = "prove graph launch";
       ctx->stages_valid = false;
     } else if (g) {
-      e = prove_body(ctx, pk, P, d_w, dom1, dom2, &where);
+      e = prove_body(ctx, pk, P, dom1, dom2, &where);
       ctx->stages_valid = true;
     } else {
-      e = prove_capture(ctx, pk, P, d_w, dom1, dom2, &where);
+      e = prove_capture(ctx, pk, P, dom1, dom2, &where);
       ctx->stages_valid = false;
     }
   }

@@ -98,11 +98,10 @@ struct cs_ctx {
   static constexpr int kAuxEvents = 9;
   cudaEvent_t aux_ev[kAuxEvents] = {nullptr};
   bool aux_ready = false;
-  // Proof launch sequences captured as CUDA graphs (prove.cu): one per key, witness buffer
-  // and scratch arena, replayed while all three are those of the capture.
+  // Proof launch sequences captured as CUDA graphs (prove.cu): one per key and scratch arena,
+  // replayed while both are those of the capture.
   struct ProveGraph {
     uint64_t pk_id = 0;
-    const void* d_w = nullptr;
     void* work = nullptr;
     size_t work_bytes = 0;
     cudaGraphExec_t exec = nullptr;  // null: the capture failed, the sequence runs launch by launch

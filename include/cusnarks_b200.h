@@ -501,9 +501,9 @@ int cs_pk_fixed_window(const cs_pk *pk, int which);
  * (groth_prover.py:1245 gen_proof; CPU sequence :575-790 and :1414-1453).
  * cs_prove: host witness and proof, synchronous.  cs_prove_device: device witness and
  * proof buffers, asynchronous on the context stream (r and s are read at call time).
- * The launch sequence after the scalar uploads is captured as a CUDA graph on the first
- * proof with a given key, witness buffer and scratch arena on a context, and replayed by
- * later proofs with the same three (one graph launch instead of ~150 API calls per proof). */
+ * The launch sequence after the scalars and the witness are in the scratch is captured as a
+ * CUDA graph on the first proof with a given key and scratch arena on a context, and replayed by
+ * later proofs with the same two (one graph launch instead of ~150 API calls per proof). */
 int cs_prove(cs_ctx *ctx, cs_pk *pk, const uint32_t *w, const uint32_t *r, const uint32_t *s,
              uint32_t *proof);
 int cs_prove_device(cs_ctx *ctx, cs_pk *pk, const uint32_t *d_w, const uint32_t *r, const uint32_t *s,
