@@ -120,26 +120,24 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   const uint32_t nb = b.nbuckets;
   const uint32_t task_len = (uint32_t)std::max(kBatchMinTask, std::min(b.task, kMaxTask));  // as the layout
   cudaError_t e;
-  if ((e = cudaMemsetAsync(counters, 0, kCtrWords * sizeof(uint32_t), st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(counts, 0, ((size_t)nb + 1) * sizeof(uint32_t), st)) != cudaSuccess) return e;
+  // counters and counts are neighbours
+  if ((e = cudaMemsetAsync(counters, 0, L.counts - L.counters + ((size_t)nb + 1) * sizeof(uint32_t), st)) != cudaSuccess)
+    return e;
   const int T = 256;
   if (b.terms) {
     k_bcount<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, counts);
     note_launch();
   }
-  if ((e = scan_exclusive_u32(counts, offsets, (size_t)nb + 1, base + L.scan, st)) != cudaSuccess) return e;
-  if ((e = cudaMemcpyAsync(counts, offsets, (size_t)nb * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st)) !=
-      cudaSuccess)
-    return e;
+  // counts becomes the scatter cursor
+  if ((e = scan_exclusive_u32(counts, offsets, (size_t)nb + 1, base + L.scan, st, counts)) != cudaSuccess) return e;
   if (b.terms) {
     k_bscatter<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, counts, entries);
     note_launch();
   }
   k_task_hist<F><<<(nb + T - 1) / T, T, 0, st>>>(offsets, nb, task_len, counters + kCtrHist, buckets);
-  k_task_bins<<<1, 32, 0, st>>>(counters + kCtrHist, task_len, counters + kCtrCursor, counters);
-  k_task_emit<F><<<(nb + T - 1) / T, T, 0, st>>>(offsets, nb, task_len, counters + kCtrCursor, tasks, counters,
-                                                  multi, b.d_jobs, b.njobs);
-  note_launch(3);
+  k_task_emit<F><<<(nb + T - 1) / T, T, 0, st>>>(offsets, nb, task_len, counters + kCtrHist, counters + kCtrCursor,
+                                                  tasks, counters, multi, b.d_jobs, b.njobs);
+  note_launch(2);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -157,13 +155,25 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(3);
   const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
-  // reduction per window group
+  // reduction: the groups that need levels of eight (and their buffers) one by one, the others'
+  // trees together (24 instances of six widths 3098 -> 2850 us, where each width took a chain of
+  // three launches)
+  BitTrees trees{};
   for (uint32_t g = 0; g < b.ngroups; g++) {
     const BatchGroup& G = b.groups[g];
     const uint32_t B = 1u << (G.c - 1);
-    reduce_buckets<F>(buckets + (size_t)G.bucket0 * XWD, B, G.windows, lv_y, lv_z, lv_y2, lv_z2,
-                      wsum + (size_t)G.window0 * XWD, nullptr, resident, st);
+    BitTrees one{};
+    const bool levels = reduce_needs_levels<F>(B, G.windows, resident);
+    BitTree t = reduce_levels<F>(buckets + (size_t)G.bucket0 * XWD, B, G.windows, lv_y, lv_z, lv_y2, lv_z2, resident, st);
+    t.wsum0 = G.window0;
+    BitTrees& T = levels ? one : trees;
+    T.t[T.count++] = t;
+    if (levels || trees.count == kMaxTrees) {
+      join_trees<F>(T, wsum, nullptr, st);
+      T.count = 0;
+    }
   }
+  if (trees.count) join_trees<F>(trees, wsum, nullptr, st);
   k_bfinish<F><<<b.njobs, 32, 0, st>>>(b.d_jobs, wsum);
   note_launch();
   return cudaGetLastError();

@@ -323,27 +323,39 @@ __global__ void k_task_hist(const uint32_t* __restrict__ offsets, uint32_t nb, u
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// Bin cursors in descending length order; counters[0] = number of tasks.
-static __global__ void k_task_bins(const uint32_t* __restrict__ hist, uint32_t task_len,
-                            uint32_t* __restrict__ cursor, uint32_t* __restrict__ counters) {
-  if (threadIdx.x != 0) return;
-  uint32_t run = 0;
-  for (int l = (int)task_len; l >= 1; l--) {
-    cursor[l] = run;
-    run += hist[l];
-  }
-  counters[0] = run;
-}
-
-// Pass 2: emit task records at their sorted positions.  Each block reserves a range per
-// length bin with one global atomic, then ranks its tasks inside it.
+// Pass 2: emit task records at their sorted positions (longest first).  Each block works out
+// where the length bins start, reserves a range per bin with one global atomic and ranks its
+// tasks inside it.  counters[0] = number of tasks.
 template <class F>
 __global__ void k_task_emit(const uint32_t* __restrict__ offsets, uint32_t nb, uint32_t task_len,
-                            uint32_t* __restrict__ cursor, Task* __restrict__ tasks,
+                            const uint32_t* __restrict__ hist, uint32_t* __restrict__ cursor, Task* __restrict__ tasks,
                             uint32_t* __restrict__ counters, Multi* __restrict__ multi,
                             const BatchJob* __restrict__ jobs = nullptr, uint32_t njobs = 0) {
-  __shared__ uint32_t cnt_s[kMaxTask + 1], base_s[kMaxTask + 1];
+  __shared__ uint32_t cnt_s[kMaxTask + 1], base_s[kMaxTask + 1], first_s[kMaxTask + 1];
   for (int i = threadIdx.x; i <= kMaxTask; i += blockDim.x) cnt_s[i] = 0;
+  if (threadIdx.x < 32) {  // bin l starts after the tasks longer than l
+    constexpr int per = (kMaxTask + 32) / 32;  // bins a lane, from kMaxTask down
+    const int top = kMaxTask - per * (int)threadIdx.x;
+    uint32_t v[per], sum = 0;
+#pragma unroll
+    for (int q = 0; q < per; q++) {
+      v[q] = top - q >= 1 ? hist[top - q] : 0u;
+      sum += v[q];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+      if ((int)threadIdx.x >= d) incl += t;
+    }
+    uint32_t run = incl - sum;
+#pragma unroll
+    for (int q = 0; q < per; q++) {
+      if (top - q >= 0) first_s[top - q] = run;
+      run += v[q];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 31) counters[0] = incl;
+  }
   __syncthreads();
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t start = 0, cnt = 0, nfull = 0, last = 0;
@@ -359,7 +371,7 @@ __global__ void k_task_emit(const uint32_t* __restrict__ offsets, uint32_t nb, u
   }
   __syncthreads();
   for (int i = threadIdx.x; i <= kMaxTask; i += blockDim.x)
-    base_s[i] = cnt_s[i] ? atomicAdd(&cursor[i], cnt_s[i]) : 0u;
+    base_s[i] = cnt_s[i] ? first_s[i] + atomicAdd(&cursor[i], cnt_s[i]) : 0u;
   __syncthreads();
   for (int i = threadIdx.x; i <= kMaxTask; i += blockDim.x) cnt_s[i] = 0;
   __syncthreads();
@@ -637,27 +649,46 @@ __global__ void __launch_bounds__(128) k_reduce_level(const uint32_t* __restrict
 // One block joins 2^lg <= 64 values in shared memory: node i of level q starts at slot i 2^q and
 // its T_j lies in slot i 2^q + 2^j, where the right half's total already is.  It writes its total
 // and T_j back to the same places, so a later stage finds the earlier bits' partial sums at the
-// same offsets of every 64 slots and adds them up (blockIdx.x: segment and window; blockIdx.y: 0 the totals, which give the
-// next bits; 1..bits the T_j; then z, whose plain sum is needed); after the last stage window w
-// has its total in slot 0 and T_j in slot 2^j.
-// Measured against the segment sums it replaces (group operations there too): see
-// reduce_buckets.
+// same offsets of every 64 slots and adds them up (blockIdx.x: bucket sets and their segments;
+// blockIdx.y: 0 the totals, which give the next bits; 1..bits the T_j; then z, whose plain sum is
+// needed); after the last stage a set has its total in slot 0 and T_j in slot 2^j.
+// The sets of all windows, and of all window widths of a batch, go through one launch a stage.
+struct BitTree {
+  uint32_t *y, *z;         // windows * 2^k values each (z may be null)
+  uint32_t k, windows;     // bits of a set's index, sets
+  uint32_t shift;          // weight of a value: 2^shift times its index
+  uint32_t block0, wsum0;  // first block of a launch, first window sum
+};
+constexpr int kMaxTrees = 24;  // widths 4..24
+struct BitTrees {
+  BitTree t[kMaxTrees];
+  int count;
+};
+CSB_DEV const BitTree& tree_of_block(const BitTrees& T) {
+  int i = 0;
+  while (i + 1 < T.count && T.t[i + 1].block0 <= blockIdx.x) i++;
+  return T.t[i];
+}
 template <class F> struct TreeGroups { static constexpr int value = 32; };
 template <> struct TreeGroups<Fq2> { static constexpr int value = 16; };  // 48 KB of shared memory
 
 template <class F>
-__global__ void __launch_bounds__(Group<F>::G* TreeGroups<F>::value, 512 / (Group<F>::G * TreeGroups<F>::value)) k_bit_tree(uint32_t* __restrict__ y,
-                                                                               uint32_t* __restrict__ z, uint32_t n,
-                                                                               int bits, int lg) {
+__global__ void __launch_bounds__(Group<F>::G* TreeGroups<F>::value, 512 / (Group<F>::G * TreeGroups<F>::value))
+    k_bit_tree(const __grid_constant__ BitTrees trees, int bits) {
   using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
   constexpr uint32_t NG = TreeGroups<F>::value, G = Gr::G;
   __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], node[64][XW];
+  const BitTree& tr = tree_of_block(trees);
+  uint32_t *y = tr.y, *z = tr.z;
+  const int lg = min(6, (int)tr.k - bits);
+  const uint32_t n = 1u << tr.k, block = blockIdx.x - tr.block0;
+  if ((int)blockIdx.y > bits && !z) return;
   const Gr grp(scr[threadIdx.x / G]);
   const uint32_t g = threadIdx.x / G, g0 = (threadIdx.x & ~31u) / G;  // this group, the warp's first
   const int role = blockIdx.y;
-  const uint32_t segs = n >> (bits + lg), seg = blockIdx.x % segs;
-  uint32_t* arr = (role <= bits ? y : z) + (size_t)(blockIdx.x / segs) * n * XW;
+  const uint32_t segs = n >> (bits + lg), seg = block % segs;
+  uint32_t* arr = (role <= bits ? y : z) + (size_t)(block / segs) * n * XW;
   const uint32_t off = role >= 1 && role <= bits ? 1u << (role - 1) : 0u;
   auto at = [&](uint32_t i) { return arr + ((size_t)((((seg << lg) + i) << bits) + off)) * XW; };
   for (uint32_t w = threadIdx.x; w < (XW / 4u) << lg; w += blockDim.x) {
@@ -684,21 +715,23 @@ __global__ void __launch_bounds__(Group<F>::G* TreeGroups<F>::value, 512 / (Grou
   }
 }
 
-// One warp per window: Z + Y + 2^shift sum_j 2^j T_j from the places k_bit_tree left them in (z
-// null: no Z), the bits in two halves at once: the upper half's Horner chain, doubled over the
-// lower bits, joins the lower's.  out: the affine result (one window), else wsum[window].
+// One warp per bucket set: Z + Y + 2^shift sum_j 2^j T_j from the places k_bit_tree left them in
+// (no Z where z is null), the bits in two halves at once: the upper half's Horner chain, doubled
+// over the lower bits, joins the lower's.  out: the affine result (one set), else wsum.
 template <class F>
-__global__ void __launch_bounds__(32) k_window_horner(const uint32_t* __restrict__ y, const uint32_t* __restrict__ z,
-                                                      uint32_t n, int bits, int shift, uint32_t* __restrict__ wsum,
-                                                      uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(32) k_window_horner(const __grid_constant__ BitTrees trees,
+                                                      uint32_t* __restrict__ wsum, uint32_t* __restrict__ out) {
   using Gr = Group<F>;
   constexpr int XW = 4 * FieldWords<F>::value;
   constexpr uint32_t G = Gr::G, NG = 32 / G;
   __shared__ __align__(16) uint32_t scr[NG][Gr::kScratch], accs[NG][XW];
+  const BitTree& tr = tree_of_block(trees);
+  const uint32_t *y = tr.y, *z = tr.z, n = 1u << tr.k, window = blockIdx.x - tr.block0;
+  const int bits = (int)tr.k, shift = (int)tr.shift;
   const Gr grp(scr[threadIdx.x / G]);
   uint32_t* acc = accs[threadIdx.x / G];
   const bool upper = ((threadIdx.x / G) & 1) != 0;
-  const uint32_t* yw = y + (size_t)blockIdx.x * n * XW;
+  const uint32_t* yw = y + (size_t)window * n * XW;
   const int s = (bits + 1) / 2, lo = upper ? s : 0;
   auto has = [&](int i) { return lo + i < bits; };
   auto T = [&](int i) { return yw + ((size_t)1 << (lo + i)) * XW; };
@@ -713,12 +746,12 @@ __global__ void __launch_bounds__(32) k_window_horner(const uint32_t* __restrict
   grp.add(acc, acc, accs[(threadIdx.x / G) | 1], !upper);
   double_times<F>(grp, acc, shift);
   grp.add(acc, acc, yw, !upper);
-  if (z) grp.add(acc, acc, z + (size_t)blockIdx.x * n * XW, !upper);
+  if (z) grp.add(acc, acc, z + (size_t)window * n * XW, !upper);
   if (threadIdx.x >= G) return;
   if (out) {
     if (threadIdx.x == 0) Gr::store_affine(out, a0);
   } else {
-    grp.store(wsum + (size_t)blockIdx.x * XW, a0);
+    grp.store(wsum + (size_t)(tr.wsum0 + window) * XW, a0);
   }
 }
 
@@ -919,9 +952,6 @@ static __global__ void k_half_counts(const uint32_t* __restrict__ off, uint32_t 
 constexpr int kCtrHist = 16, kCtrCursor = 128, kCtrWords = 256;
 static_assert(kCtrHist + kMaxTask + 1 <= kCtrCursor && kCtrCursor + kMaxTask + 1 <= kCtrWords,
               "task-length bins must not overlap");
-// the reduction runs eight buckets per thread while the remaining values times a group's lanes
-// exceed this many times the resident threads
-constexpr uint64_t kTreeFill = 16;
 
 struct Layout {
   size_t counts, offsets, entries, tasks, multi, partials, buckets, lv_y, lv_z, lv_y2, lv_z2, wsum,
@@ -1030,33 +1060,64 @@ int accumulate_grid(int dev, int sms) {
   return b * sms;
 }
 
-// The window sums of WR bucket sets of B = 2^(c-1) buckets each (overwritten), to wsum, or the
-// affine result of a single set to out.  Levels of eight buckets per thread (least work) while
-// the rest would fill the resident threads' groups several times over, then the bit tree.
+// The bucket sums of WR sets of B = 2^(c-1) buckets each (overwritten) as a tree to join: levels
+// of eight buckets per thread (least work, and what fills the GPU best) come first while the
+// values would fill the resident threads' groups many times over.
+// Measured (us): 22 sets of 2048 over Fq2, levels 252 + 61, tree 172; 2^19 buckets over Fq, levels
+// 268 + 97, tree alone 500.
+template <class F> struct TreeFill { static constexpr uint64_t value = 16; };
+template <> struct TreeFill<Fq2> { static constexpr uint64_t value = 32; };
 template <class F>
-void reduce_buckets(uint32_t* buckets, uint32_t B, uint32_t WR, uint32_t* lv_y, uint32_t* lv_z, uint32_t* lv_y2,
-                    uint32_t* lv_z2, uint32_t* wsum, uint32_t* out, uint64_t resident, cudaStream_t st) {
-  uint32_t *y = buckets, *z = nullptr, n = B;
+bool reduce_needs_levels(uint32_t n, uint32_t WR, uint64_t resident) {
+  return n >= 8 && (uint64_t)n * WR * Group<F>::G > TreeFill<F>::value * resident;
+}
+template <class F>
+BitTree reduce_levels(uint32_t* buckets, uint32_t B, uint32_t WR, uint32_t* lv_y, uint32_t* lv_z, uint32_t* lv_y2,
+                      uint32_t* lv_z2, uint64_t resident, cudaStream_t st) {
+  BitTree t{buckets, nullptr, 0, WR, 0, 0, 0};
+  uint32_t n = B;
   int level = 0;
-  while (n >= 8 && (uint64_t)n * WR * Group<F>::G > kTreeFill * resident) {
+  for (; reduce_needs_levels<F>(n, WR, resident); level++) {
     const uint32_t nout = n / 8;
     uint32_t *yo = level % 2 ? lv_y2 : lv_y, *zo = level % 2 ? lv_z2 : lv_z;
-    k_reduce_level<F><<<(uint32_t)(((uint64_t)WR * nout + 127) / 128), 128, 0, st>>>(y, z, n, nout, (int)WR, level, yo, zo);
+    k_reduce_level<F><<<(uint32_t)(((uint64_t)WR * nout + 127) / 128), 128, 0, st>>>(t.y, t.z, n, nout, (int)WR, level, yo,
+                                                                                      zo);
     note_launch();
-    y = yo;
-    z = zo;
+    t.y = yo;
+    t.z = zo;
     n = nout;
-    level++;
   }
-  int k = 0;
-  while ((1u << k) < n) k++;
-  for (int bits = 0; bits < k; bits += 6) {
-    const int lg = std::min(6, k - bits);
-    k_bit_tree<F><<<dim3(WR * (n >> (bits + lg)), 1 + bits + (z ? 1 : 0)), Group<F>::G * TreeGroups<F>::value, 0, st>>>(
-        y, z, n, bits, lg);
+  t.shift = 3 * level;
+  while ((1u << t.k) < n) t.k++;
+  return t;
+}
+// Joins the trees: their window sums to wsum, or the affine result of a single set to out.
+template <class F>
+void join_trees(BitTrees& T, uint32_t* wsum, uint32_t* out, cudaStream_t st) {
+  uint32_t kmax = 0;
+  bool any_z = false;
+  for (int i = 0; i < T.count; i++) {
+    kmax = std::max(kmax, T.t[i].k);
+    any_z |= T.t[i].z != nullptr;
+  }
+  for (uint32_t bits = 0; bits < kmax; bits += 6) {
+    BitTrees S{};  // the trees that still have bits to join
+    uint32_t blocks = 0;
+    for (int i = 0; i < T.count; i++) {
+      if (T.t[i].k <= bits) continue;
+      BitTree& t = S.t[S.count++] = T.t[i];
+      t.block0 = blocks;
+      blocks += t.windows << (t.k - bits - std::min(6u, t.k - bits));
+    }
+    k_bit_tree<F><<<dim3(blocks, 1 + bits + (any_z ? 1 : 0)), Group<F>::G * TreeGroups<F>::value, 0, st>>>(S, (int)bits);
     note_launch();
   }
-  k_window_horner<F><<<WR, 32, 0, st>>>(y, z, n, k, 3 * level, wsum, out);
+  uint32_t blocks = 0;
+  for (int i = 0; i < T.count; i++) {
+    T.t[i].block0 = blocks;
+    blocks += T.t[i].windows;
+  }
+  k_window_horner<F><<<blocks, 32, 0, st>>>(T, wsum, out);
   note_launch();
 }
 
@@ -1142,17 +1203,16 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
       note_launch();
     }
   }
-  if ((e = cudaMemsetAsync(counters, 0, kCtrWords * sizeof(uint32_t), st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(counts, 0, (nb + 1) * sizeof(uint32_t), st)) != cudaSuccess) return e;
+  // counters and counts are neighbours
+  if ((e = cudaMemsetAsync(counters, 0, L.counts - L.counters + ((size_t)nb + 1) * sizeof(uint32_t), st)) != cudaSuccess)
+    return e;
   if (glv)
     k_count_glv<F><<<(n_in + T - 1) / T, T, 0, st>>>(glv_s, n_in, c, W, counts);
   else
     k_count<F, FIXED><<<(n + T - 1) / T, T, 0, st>>>(d_scalars, d_points, n, c, W, counts);
   note_launch();
-  if ((e = scan_exclusive_u32(counts, offsets, nb + 1, scan_tmp, st)) != cudaSuccess) return e;
-  // counts is reused as the scatter cursor
-  if ((e = cudaMemcpyAsync(counts, offsets, nb * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-    return e;
+  // counts becomes the scatter cursor
+  if ((e = scan_exclusive_u32(counts, offsets, (size_t)nb + 1, scan_tmp, st, counts)) != cudaSuccess) return e;
   if (glv)
     k_scatter_glv<F><<<(n_in + T - 1) / T, T, 0, st>>>(glv_s, n_in, c, W, counts, entries);
   else
@@ -1193,10 +1253,8 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
   }
   k_task_hist<F><<<(nb + T - 1) / T, T, 0, st>>>(acc_off, nb, task_len, counters + kCtrHist, buckets);
   note_launch();
-  k_task_bins<<<1, 32, 0, st>>>(counters + kCtrHist, task_len, counters + kCtrCursor, counters);
-  note_launch();
-  k_task_emit<F><<<(nb + T - 1) / T, T, 0, st>>>(acc_off, nb, task_len, counters + kCtrCursor, tasks,
-                                                  counters, multi);
+  k_task_emit<F><<<(nb + T - 1) / T, T, 0, st>>>(acc_off, nb, task_len, counters + kCtrHist, counters + kCtrCursor,
+                                                  tasks, counters, multi);
   note_launch();
   if (cfg.acc_start) cudaEventRecord(cfg.acc_start, st);
   if (latency_mode)
@@ -1222,8 +1280,9 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
     k_add_buckets<F><<<(B + 127) / 128, 128, 0, st>>>(buckets, cfg.bucket_add, B);
     note_launch();
   }
-  reduce_buckets<F>(buckets, B, (uint32_t)WR, lv_y, lv_z, lv_y2, lv_z2, cfg.xyzz_out && WR == 1 ? cfg.xyzz_out : wsum,
-                    WR == 1 && !cfg.xyzz_out ? d_out : nullptr, resident, st);
+  BitTrees trees{};
+  trees.t[trees.count++] = reduce_levels<F>(buckets, B, (uint32_t)WR, lv_y, lv_z, lv_y2, lv_z2, resident, st);
+  join_trees<F>(trees, cfg.xyzz_out && WR == 1 ? cfg.xyzz_out : wsum, WR == 1 && !cfg.xyzz_out ? d_out : nullptr, st);
   if (WR > 1) {
     k_finish<F><<<1, 32, 0, st>>>(wsum, WR, c, d_out, cfg.xyzz_out);
     note_launch();

@@ -123,7 +123,8 @@ __global__ void k_wire_counts2(const uint32_t* __restrict__ mpoly, uint32_t n_wi
 }  // namespace
 
 namespace csb {
-cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, void* tmp, cudaStream_t stream);
+cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, void* tmp, cudaStream_t stream,
+                               uint32_t* out2 = nullptr);
 size_t scan_workspace_bytes(size_t n);
 }  // namespace csb
 
