@@ -34,7 +34,7 @@ int pick_window(int dev, int ec2, uint32_t n) {
     const int w = g_tuned[dev][ec2 ? 1 : 0][ceil_log2(n < 1 ? 1 : n)];
     if (w) return w;
   }
-  return csb::msm_window_model(n ? n : 1, false);  // batch instances sort full scalars
+  return csb::msm_default_window(n ? n : 1, ec2 != 0);
 }
 
 // Pseudo-random limbs for timing runs (splitmix-style hash); top limb masked below 2^253 so
@@ -103,10 +103,14 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
   std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t x, uint32_t y) { return win[x] < win[y]; });
   uint64_t terms = 0, buckets = 0, entries = 0, windows = 0;
   uint64_t lv = 0, lv2 = 0;
+  bool any_glv = false;
   for (uint32_t k = 0; k < njobs; k++) {
     const BatchSpec& j = jobs[b->order[k]];
     const int c = win[b->order[k]];
-    const uint32_t W = 254 / c + 1;
+    // generic G1 instances split their scalars as single MSMs do: half the bucket sets and half
+    // the Horner chain (24 instances of 2^10..2^16 terms: 2.85 -> 2.45 ms)
+    const bool glv = !ec2 && !j.fixed && j.n < (1u << 30);
+    const uint32_t W = glv ? (128 + c - 1) / c : 254 / c + 1;
     const uint32_t sets = j.fixed ? 1u : W;
     BatchJob bj{};
     bj.scalars = j.scalars;
@@ -117,6 +121,7 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
     bj.W = W;
     bj.fixed = j.fixed ? 1u : 0u;
     bj.sets = sets;
+    bj.glv = glv ? 1u : 0u;
     bj.term0 = (uint32_t)terms;
     bj.bucket0 = (uint32_t)buckets;
     bj.window0 = (uint32_t)windows;
@@ -125,7 +130,8 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
     b->groups.back().windows += sets;
     terms += j.n;
     buckets += (uint64_t)sets << (c - 1);
-    entries += (uint64_t)j.n * W;
+    entries += (uint64_t)j.n * W * (glv ? 2 : 1);
+    any_glv |= glv;
     windows += sets;
     b->jobs.push_back(bj);
   }
@@ -142,6 +148,7 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
   P.nbuckets = (uint32_t)buckets;
   P.nentries = entries;
   P.nwindows = (uint32_t)windows;
+  P.glv = any_glv;
   P.lv_points = lv;
   P.lv2_points = lv2;
   P.groups = b->groups.data();
@@ -269,17 +276,14 @@ int cs_msm_autotune(cs_ctx* ctx, int ec2, uint32_t log_min, uint32_t log_max, in
     if (e == cudaSuccess) e = cudaEventCreate(&z);
     for (uint32_t L = log_min; L <= log_max && e == cudaSuccess; L++) {
       const uint32_t n = 1u << L;
-      // the form a batch instance runs: full scalars (single G1 MSMs split them by GLV and
-      // keep the cost model's window)
-      const int c0 = csb::msm_window_model(n, false);
+      const int c0 = csb::msm_default_window(n, ec2 != 0);
       float best = 1e30f;
       int bw = c0;
       for (int c = std::max(4, c0 - 2); c <= std::min(22, c0 + 2) && e == cudaSuccess; c++) {
-        e = ctx->work.reserve(csb::msm_workspace_bytes(n, c, ec2 != 0, -1, 0), ctx->stream);
+        e = ctx->work.reserve(csb::msm_workspace_bytes(n, c, ec2 != 0), ctx->stream);
         if (e != cudaSuccess) break;
         csb::MsmConfig cfg;
         cfg.c = c;
-        cfg.glv = 0;
         float t_best = 1e30f;
         for (int rep = 0; rep < 3 && e == cudaSuccess; rep++) {
           cudaEventRecord(a, ctx->stream);

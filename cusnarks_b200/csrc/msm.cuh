@@ -41,12 +41,13 @@ namespace csb {
 // contiguous bucket range).
 // A batch instance.  fixed = 0: points holds n points, W bucket sets (one per window).
 // fixed = 1: points is a fixed-base table T[j n + i] = 2^(c j) P_i of W windows, one bucket set
-// (entries are table indices), no window Horner.  sets: bucket sets (W or 1).
+// (entries are table indices), no window Horner.  sets: bucket sets (W or 1).  glv: a generic G1
+// instance, its scalars split by the endomorphism as a single MSM's are.
 struct BatchJob {
   const uint32_t* scalars;
   const uint32_t* points;
   uint32_t* out;
-  uint32_t n, c, W, bucket0, window0, term0, fixed, sets;
+  uint32_t n, c, W, bucket0, window0, term0, fixed, sets, glv;
 };
 
 // A group of batch instances sharing one window c: buckets [bucket0, bucket0 + windows * B),
@@ -68,6 +69,7 @@ struct MsmBatch {
   uint64_t lv_points = 0, lv2_points = 0;  // max over groups of W*(2^(c-1)/8+1), W*(.../64+1)
   const BatchGroup* groups = nullptr;  // host array
   uint32_t ngroups = 0;
+  bool glv = false;        // some instance is split (its side arrays are sized by terms)
   int task = 64;           // entries per accumulation task, kBatchMinTask..64 (set by the builder)
 };
 constexpr int kBatchMinTask = 8;

@@ -35,16 +35,37 @@ CSB_DEV uint32_t job_of_term(const BatchJob* jobs, uint32_t njobs, uint32_t t) {
   return lo;
 }
 
+// Splits the terms of the split instances: halves to s2, beta x to phix, at the global term.
+template <class F>
+__global__ void k_bprep(const BatchJob* __restrict__ jobs, uint32_t njobs, uint32_t terms, uint32_t* __restrict__ s2,
+                        uint32_t* __restrict__ phix) {
+  constexpr int PW = 2 * FieldWords<F>::value;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= terms) return;
+  const BatchJob jb = jobs[job_of_term(jobs, njobs, t)];
+  if (!jb.glv) return;
+  const uint32_t i = t - jb.term0;
+  glv_prep_term<F>(jb.scalars + (size_t)i * 8, jb.points + (size_t)i * PW, s2 + (size_t)t * 8, phix + (size_t)t * 8);
+}
+
 template <class F>
 __global__ void k_bcount(const BatchJob* __restrict__ jobs, uint32_t njobs, uint32_t terms,
-                         uint32_t* __restrict__ counts) {
+                         const uint32_t* __restrict__ s2, uint32_t* __restrict__ counts) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= terms) return;
   const BatchJob jb = jobs[job_of_term(jobs, njobs, t)];
   const uint32_t i = t - jb.term0;
   uint32_t k[8];
-  if (!load_scalar<F>(jb.scalars, jb.points, i, k)) return;
   const uint32_t B = 1u << (jb.c - 1);
+  if (jb.glv) {
+    ld_limbs8(k, s2 + (size_t)t * 8);
+    for_each_glv_digit(k, (int)jb.c, (int)jb.W, [&](int, int j, uint32_t mag, bool) {
+      const size_t b = jb.bucket0 + (size_t)j * B + (mag - 1);
+      if (j == 0) claim_shared(counts, b); else atomicAdd(&counts[b], 1u);
+    });
+    return;
+  }
+  if (!load_scalar<F>(jb.scalars, jb.points, i, k)) return;
   for_each_digit(k, (int)jb.c, (int)jb.W, [&](int j, uint32_t mag, bool) {
     const size_t b = jb.bucket0 + (jb.fixed ? 0 : (size_t)j * B) + (mag - 1);
     if (j == 0) claim_shared(counts, b); else atomicAdd(&counts[b], 1u);
@@ -53,12 +74,18 @@ __global__ void k_bcount(const BatchJob* __restrict__ jobs, uint32_t njobs, uint
 
 template <class F>
 __global__ void k_bscatter(const BatchJob* __restrict__ jobs, uint32_t njobs, uint32_t terms,
-                           uint32_t* __restrict__ cursor, uint32_t* __restrict__ entries) {
+                           const uint32_t* __restrict__ s2, uint32_t* __restrict__ cursor,
+                           uint32_t* __restrict__ entries) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= terms) return;
   const BatchJob jb = jobs[job_of_term(jobs, njobs, t)];
   const uint32_t i = t - jb.term0;
   uint32_t k[8];
+  if (jb.glv) {
+    ld_limbs8(k, s2 + (size_t)t * 8);
+    scatter_glv_term(k, i, (int)jb.c, (int)jb.W, jb.bucket0, cursor, entries);
+    return;
+  }
   if (!load_scalar<F>(jb.scalars, jb.points, i, k)) return;
   const uint32_t B = 1u << (jb.c - 1);
   scatter_digits(k, (int)jb.c, (int)jb.W, cursor, entries,
@@ -76,7 +103,7 @@ __global__ void __launch_bounds__(32) k_bfinish(const BatchJob* __restrict__ job
 
 struct BatchLayout {
   size_t counters, counts, offsets, entries, tasks, multi, partials, buckets, lv_y, lv_z, lv_y2, lv_z2, wsum,
-      scan, total;
+      glv_s, glv_p, scan, total;
 };
 
 inline BatchLayout batch_layout(const MsmBatch& b, int xyzz_bytes) {
@@ -98,6 +125,12 @@ inline BatchLayout batch_layout(const MsmBatch& b, int xyzz_bytes) {
   L.lv_y2 = o;    o = align256(o + lv2 * xyzz_bytes);
   L.lv_z2 = o;    o = align256(o + lv2 * xyzz_bytes);
   L.wsum = o;     o = align256(o + (size_t)b.nwindows * xyzz_bytes);
+  L.glv_s = L.glv_p = o;
+  if (b.glv) {
+    o = align256(o + (size_t)b.terms * 32);
+    L.glv_p = o;
+    o = align256(o + (size_t)b.terms * 32);
+  }
   L.scan = o;
   L.total = o + scan_workspace_bytes(nb + 1);
   return L;
@@ -124,14 +157,21 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   if ((e = cudaMemsetAsync(counters, 0, L.counts - L.counters + ((size_t)nb + 1) * sizeof(uint32_t), st)) != cudaSuccess)
     return e;
   const int T = 256;
+  uint32_t *glv_s = at(L.glv_s), *phix = b.glv ? at(L.glv_p) : nullptr;
+  if constexpr (FieldWords<F>::value == 8) {
+    if (b.glv && b.terms) {
+      k_bprep<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, glv_s, phix);
+      note_launch();
+    }
+  }
   if (b.terms) {
-    k_bcount<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, counts);
+    k_bcount<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, glv_s, counts);
     note_launch();
   }
   // counts becomes the scatter cursor
   if ((e = scan_exclusive_u32(counts, offsets, (size_t)nb + 1, base + L.scan, st, counts)) != cudaSuccess) return e;
   if (b.terms) {
-    k_bscatter<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, counts, entries);
+    k_bscatter<F><<<(b.terms + T - 1) / T, T, 0, st>>>(b.d_jobs, b.njobs, b.terms, glv_s, counts, entries);
     note_launch();
   }
   k_task_hist<F><<<(nb + T - 1) / T, T, 0, st>>>(offsets, nb, task_len, counters + kCtrHist, buckets);
@@ -147,10 +187,11 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   const uint64_t resident_threads = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
   const bool latency_mode = ((uint64_t)nb + b.nentries / task_len + 1) * 4 <= resident_threads * 4;
   if (latency_mode)
-    k_accumulate_group<F><<<sms * 8, 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets, partials, b.d_jobs);
+    k_accumulate_group<F><<<sms * 8, 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets, partials, b.d_jobs,
+                                                    phix);
   else
     k_accumulate<F><<<accumulate_grid<F>(dev, sms), 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets,
-                                                             partials, b.d_jobs);
+                                                             partials, b.d_jobs, phix);
   k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, nb, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(3);

@@ -183,15 +183,10 @@ __global__ void k_scatter(const uint32_t* __restrict__ scalars, const uint32_t* 
 // points themselves are not copied: an entry of the k2 half carries PHI_BIT and reads x from
 // phix and y from P_i, so the gathered set stays the n input points plus n x-coordinates.
 template <class F>
-__global__ void k_glv_prep(const uint32_t* __restrict__ scalars, const uint32_t* __restrict__ points, uint32_t n,
-                           uint32_t* __restrict__ s2, uint32_t* __restrict__ phix) {
-  constexpr int PW = 2 * FieldWords<F>::value;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+CSB_DEV void glv_prep_term(const uint32_t* scalar, const uint32_t* P, uint32_t* s2, uint32_t* phix) {
   uint32_t k[8];
-  ld_limbs8(k, scalars + (size_t)i * 8);
+  ld_limbs8(k, scalar);
   scalar_reduce(k);
-  const uint32_t* P = points + (size_t)i * PW;
   uint32_t k1[4] = {0, 0, 0, 0}, k2[4] = {0, 0, 0, 0}, neg1 = 0, neg2 = 0;
   const bool zero = (k[0] | k[1] | k[2] | k[3] | k[4] | k[5] | k[6] | k[7]) == 0;
   if (!zero && !point_is_inf<F>(P)) {
@@ -199,13 +194,21 @@ __global__ void k_glv_prep(const uint32_t* __restrict__ scalars, const uint32_t*
                             k[6] | (uint64_t)k[7] << 32};
     glv::split_reduced(kk, k1, &neg1, k2, &neg2);
   }
-  uint4* o = reinterpret_cast<uint4*>(s2 + (size_t)i * 8);
+  uint4* o = reinterpret_cast<uint4*>(s2);
   o[0] = make_uint4(k1[0], k1[1], k1[2], k1[3] | (neg1 << 31));
   o[1] = make_uint4(k2[0], k2[1], k2[2], k2[3] | (neg2 << 31));
   F x, beta;
   ld_field(x, P);
   glv::beta_mont(beta.v);
-  st_field(phix + (size_t)i * 8, x * beta);
+  st_field(phix, x * beta);
+}
+template <class F>
+__global__ void k_glv_prep(const uint32_t* __restrict__ scalars, const uint32_t* __restrict__ points, uint32_t n,
+                           uint32_t* __restrict__ s2, uint32_t* __restrict__ phix) {
+  constexpr int PW = 2 * FieldWords<F>::value;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  glv_prep_term<F>(scalars + (size_t)i * 8, points + (size_t)i * PW, s2 + (size_t)i * 8, phix + (size_t)i * 8);
 }
 
 // Digits of both halves of a split term: f(half, window, |d|, negative), the half's sign
@@ -217,6 +220,19 @@ CSB_DEV void for_each_glv_digit(const uint32_t (&t)[8], int c, int W, Fn f) {
     const uint32_t k[8] = {t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3] & 0x7fffffffu, 0u, 0u, 0u, 0u};
     const bool sgn = (t[4 * h + 3] >> 31) != 0;
     for_each_digit(k, c, W, [&](int j, uint32_t mag, bool neg) { f(h, j, mag, neg != sgn); });
+  }
+}
+
+// Places a split term's entries; its buckets start at bucket0.
+CSB_DEV void scatter_glv_term(const uint32_t (&t)[8], uint32_t i, int c, int W, uint32_t bucket0, uint32_t* cursor,
+                              uint32_t* entries) {
+  const uint32_t B = 1u << (c - 1);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const uint32_t k[8] = {t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3] & 0x7fffffffu, 0u, 0u, 0u, 0u};
+    const bool sgn = (t[4 * h + 3] >> 31) != 0;
+    scatter_digits(k, c, W, cursor, entries, [&](int j, uint32_t mag) { return bucket0 + (size_t)j * B + (mag - 1); },
+                   [&](int, bool neg) { return i | (h ? PHI_BIT : 0u) | (neg != sgn ? NEG_BIT : 0u); });
   }
 }
 
@@ -240,14 +256,7 @@ __global__ void k_scatter_glv(const uint32_t* __restrict__ s2, uint32_t n, int c
   if (i >= n) return;
   uint32_t t[8];
   ld_limbs8(t, s2 + (size_t)i * 8);
-  const uint32_t B = 1u << (c - 1);
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const uint32_t k[8] = {t[4 * h], t[4 * h + 1], t[4 * h + 2], t[4 * h + 3] & 0x7fffffffu, 0u, 0u, 0u, 0u};
-    const bool sgn = (t[4 * h + 3] >> 31) != 0;
-    scatter_digits(k, c, W, cursor, entries, [&](int j, uint32_t mag) { return (size_t)j * B + (mag - 1); },
-                   [&](int, bool neg) { return i | (h ? PHI_BIT : 0u) | (neg != sgn ? NEG_BIT : 0u); });
-  }
+  scatter_glv_term(t, i, c, W, 0, cursor, entries);
 }
 
 // The base of an entry: P_i, or phi(P_i) = (phix[i], y_i) for a GLV k2 entry (phix given).
@@ -268,6 +277,11 @@ CSB_DEV Affine<F> ld_entry_point(const uint32_t* base, const uint32_t* phix, uin
   } else {
     return ld_affine<F>(base + (size_t)(ent & ~NEG_BIT) * PW);
   }
+}
+
+// A batch's side array of beta x holds its terms' in order (unused where an instance is not split).
+CSB_DEV const uint32_t* job_phix(const BatchJob& jb, const uint32_t* phix) {
+  return jb.glv ? phix + (size_t)jb.term0 * 8 : nullptr;
 }
 
 // Task record: entries [start, start+len) summed into dst.  dst < nb: bucket index;
@@ -451,12 +465,13 @@ __global__ void __launch_bounds__(128, AccMinBlocks<F>::value) k_accumulate(cons
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntasks; t += gridDim.x * blockDim.x) {
     const Task tk = tasks[t];
     const uint32_t* base = jobs ? jobs[tk.job].points : points;
+    const uint32_t* px = jobs ? job_phix(jobs[tk.job], phix) : phix;
     XYZZ<F> acc = XYZZ<F>::inf();
     if (entries) {
 #pragma unroll 1
       for (uint32_t e = 0; e < tk.len; e++) {
         const uint32_t ent = entries[tk.start + e];
-        Affine<F> p = ld_entry_point<F>(base, phix, ent);
+        Affine<F> p = ld_entry_point<F>(base, px, ent);
         if (ent & NEG_BIT) p.y = p.y.neg();
         acc = madd_acc(acc, p);
       }
@@ -498,6 +513,7 @@ __global__ void __launch_bounds__(128, 4) k_accumulate_group(
     const bool valid = t < ntasks;
     const Task tk = valid ? tasks[t] : Task{0, 0, 0, 0};
     const uint32_t* pts = jobs && valid ? jobs[tk.job].points : points;  // read only where live
+    const uint32_t* px = jobs ? (valid ? job_phix(jobs[tk.job], phix) : nullptr) : phix;
     const uint32_t steps = __reduce_max_sync(0xffffffffu, tk.len);
     grp.load(acc, nullptr, false);
 #pragma unroll 1
@@ -507,9 +523,9 @@ __global__ void __launch_bounds__(128, 4) k_accumulate_group(
       bool neg = false;
       if (live) {
         const uint32_t ent = entries[tk.start + e];
-        const uint32_t i = ent & ~(NEG_BIT | (phix ? PHI_BIT : 0u));
+        const uint32_t i = ent & ~(NEG_BIT | (px ? PHI_BIT : 0u));
         qy = pts + (size_t)i * PW + FW;
-        qx = FW == 8 && phix && (ent & PHI_BIT) ? phix + (size_t)i * FW : pts + (size_t)i * PW;
+        qx = FW == 8 && px && (ent & PHI_BIT) ? px + (size_t)i * FW : pts + (size_t)i * PW;
         neg = (ent & NEG_BIT) != 0;
       }
       grp.madd(acc, acc, qx, qy, neg, live);
