@@ -98,9 +98,12 @@ CSB_DEV Block pass_block(const Pass& a) {
 // Throughput form (2^22 points 0.89 ms, 1.05 ms with one stage a barrier and values reduced below r
 // after each; bound by the products, 0.68 ms at the GPU's rate): a thread takes four elements through two stages at a time, so a pass
 // crosses shared memory and the barrier (S - 1) / 2 times; the first stages read from and
-// the last write to global memory directly.  An odd S starts with one single stage.  Three
-// blocks a SM (84 registers) gain 2 % from 2^20 on and lose 5 % at 2^17 to 2^19.
-__global__ void __launch_bounds__(kThreads, 2) k_ntt_pass4(const Pass a) {
+// the last write to global memory directly.  An odd S starts with one single stage.
+// BLOCKS resident blocks a SM: three (84 registers) from 2^20 points on, where there are blocks
+// enough to keep them full (2^22 893 against 868 us, H step of 2^20 1372 / 1326), two below (H
+// step of 2^18 342 against 363).
+template <int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS) k_ntt_pass4(const Pass a) {
   extern __shared__ uint4 sm[];
   const uint32_t cnt = 1u << a.S, s0 = a.s0;
   const Tile tile{sm, sm + cnt};
@@ -283,8 +286,9 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
     q.load = (int)a.load;
     q.canon = last && !a.lazy_out;
     const dim3 grid(1u << (L - S), a.batch, a.count);
+    auto* pass4 = L >= 20 ? k_ntt_pass4<3> : k_ntt_pass4<2>;
     if ((32u << S) > 48u * 1024) {  // above the default limit of a block's shared memory
-      const cudaError_t e = cudaFuncSetAttribute(latency ? (const void*)k_ntt_pass2 : (const void*)k_ntt_pass4,
+      const cudaError_t e = cudaFuncSetAttribute(latency ? (const void*)k_ntt_pass2 : (const void*)pass4,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 32 << S);
       if (e != cudaSuccess) return e;
     }
@@ -292,7 +296,7 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
       k_ntt_pass2<<<grid, 1u << (S - 1), (1u << S) * 32, st>>>(q);
     } else {
       const unsigned threads = (1u << (S - 2)) < (unsigned)kThreads ? (1u << (S - 2)) : (unsigned)kThreads;
-      k_ntt_pass4<<<grid, threads, (1u << S) * 32, st>>>(q);
+      pass4<<<grid, threads, (1u << S) * 32, st>>>(q);
     }
     note_launch();
     s0 += S;
