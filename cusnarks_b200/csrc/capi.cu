@@ -22,7 +22,7 @@ unsigned long long thread_launches() { return t_launches; }
 
 
 // Auxiliary streams of the prove pipeline: aux[0..3] carry the A, B1, B2 (G2) and C MSMs,
-// aux_h the QAP -> H step -> H MSM chain.  Priorities (lower number = higher priority)
+// aux_h the QAP -> H step -> H MSM chain, aux_s the MSM of s pi_A where that is one.  Priorities (lower number = higher priority)
 // decide which MSM's blocks the SMs take first when several are ready.
 cudaError_t ctx_aux_init(cs_ctx* ctx) {
   if (ctx->aux_ready) return cudaSuccess;
@@ -33,6 +33,7 @@ cudaError_t ctx_aux_init(cs_ctx* ctx) {
   for (int i = 0; i < 4 && e == cudaSuccess; i++)
     if (!ctx->aux[i]) e = cudaStreamCreateWithPriority(&ctx->aux[i], cudaStreamNonBlocking, prio[i]);
   if (e == cudaSuccess && !ctx->aux_h) e = cudaStreamCreateWithPriority(&ctx->aux_h, cudaStreamNonBlocking, prio_h);
+  if (e == cudaSuccess && !ctx->aux_s) e = cudaStreamCreateWithPriority(&ctx->aux_s, cudaStreamNonBlocking, least);
   for (int i = 0; i < cs_ctx::kAuxEvents && e == cudaSuccess; i++)
     if (!ctx->aux_ev[i]) e = cudaEventCreate(&ctx->aux_ev[i]);  // timed: prove stage times
   if (e == cudaSuccess) ctx->aux_ready = true;
@@ -186,6 +187,7 @@ void cs_ctx_destroy(cs_ctx* ctx) {
   for (int i = 0; i < 4; i++)
     if (ctx->aux[i]) { cudaStreamSynchronize(ctx->aux[i]); cudaStreamDestroy(ctx->aux[i]); }
   if (ctx->aux_h) { cudaStreamSynchronize(ctx->aux_h); cudaStreamDestroy(ctx->aux_h); }
+  if (ctx->aux_s) { cudaStreamSynchronize(ctx->aux_s); cudaStreamDestroy(ctx->aux_s); }
   for (int i = 0; i < cs_ctx::kAuxEvents; i++)
     if (ctx->aux_ev[i]) cudaEventDestroy(ctx->aux_ev[i]);
   delete ctx;

@@ -106,6 +106,18 @@ __global__ void k_set_tail(uint32_t* __restrict__ scalars, uint32_t n, const uin
   }
 }
 
+// wS = s wA and wR = r wB (normal form, below the modulus): the scalars whose MSMs over the A and
+// B1 bases are s pi_A and r pi_B1.
+__global__ void k_scaled_scalars(const uint32_t* __restrict__ wA, const uint32_t* __restrict__ wB, uint32_t n,
+                                 const uint32_t* __restrict__ rs, uint32_t* __restrict__ wS, uint32_t* __restrict__ wR) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const Fr r = ld_fp<ModR>(rs).to_mont(), s = ld_fp<ModR>(rs + 8).to_mont();
+  // the scalar on the right may be any 256-bit value
+  st_fp<ModR>(wS + (size_t)i * 8, s * ld_fp<ModR>(wA + (size_t)i * 8));
+  st_fp<ModR>(wR + (size_t)i * 8, r * ld_fp<ModR>(wB + (size_t)i * 8));
+}
+
 // dst = -(r s) mod r_field, normal form (the reference's montmult_neg_h(r_mont, s))
 __global__ void k_neg_rs(const uint32_t* __restrict__ r, const uint32_t* __restrict__ s, uint32_t* __restrict__ dst) {
   if (threadIdx.x != 0) return;
@@ -249,12 +261,19 @@ uint32_t ilog2_exact(uint32_t m) {
 
 // Layout of the per-call prove scratch.
 struct ProvePlan {
-  size_t wA, wB, pA, pB, M, hscr, ms_a, ms_b1, ms_b2, ms_c, ms_h, pts, rs, cbk, total;
+  size_t wA, wB, wS, wR, pA, pB, M, hscr, ms_a, ms_b1, ms_b2, ms_c, ms_h, ms_s, pts, rs, cbk, total;
   size_t bytes_a, bytes_b1, bytes_b2, bytes_c, bytes_h;
   // C and H share one bucket reduction: both fixed-base with the same window, C's buckets
   // (cbk) folded into H's before H reduces (pi_C only needs their sum)
   bool share_ch;
+  // s pi_A and r pi_B1 as MSMs of scaled scalars (the second instead of pi_B1, which nothing
+  // else needs) rather than scalar multiplications of the finished sums
+  bool scaled;
 };
+// Up to this domain a proof is a handful of latency chains on a mostly idle GPU, and one more MSM
+// beside them costs less than 127 doublings after one (us, multiplication / MSM: 2^12 from host
+// memory 654 / 583; alone, from the device, 2^13 886 / 868, 2^14 844 / 887).
+constexpr uint32_t kScaledMaxDomain = 1u << 13;
 
 ProvePlan plan_prove(const cs_pk* pk) {
   ProvePlan P{};
@@ -276,10 +295,14 @@ ProvePlan plan_prove(const cs_pk* pk) {
   size_t o = 0;
   P.wA = o; o += al256((nv + 2) * 32);
   P.wB = o; o += al256((nv + 2) * 32);
+  P.scaled = pk->has_fixed() && pk->m <= kScaledMaxDomain;
+  P.wS = o; if (P.scaled) o += al256((nv + 2) * 32);
+  P.wR = o; if (P.scaled) o += al256((nv + 2) * 32);
   P.pA = o; o += al256(m * 32);
   P.pB = o; o += al256(m * 32);
   P.M = o; o += al256(2 * m * 32);
   P.hscr = o; o += al256(4 * m * 32);
+  P.ms_s = o; if (P.scaled) o += al256(P.bytes_a);
   P.ms_a = o; o += al256(P.bytes_a);
   P.ms_b1 = o; o += al256(P.bytes_b1);
   P.ms_b2 = o; o += al256(P.bytes_b2);
@@ -318,6 +341,10 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1,
   k_set_tail<<<1, 32, 0, s0>>>(wB, nv, rs + 8);
   k_neg_rs<<<1, 32, 0, s0>>>(rs, rs + 8, rs + 16);
   note_launch(3);
+  if (P.scaled) {
+    k_scaled_scalars<<<(nv + 2 + 127) / 128, 128, 0, s0>>>(wA, wB, nv + 2, rs, at(P.wS), at(P.wR));
+    note_launch();
+  }
   cudaEventRecord(ev_w, s0);
   // witness MSMs on the auxiliary streams
   cudaStream_t sa = ctx->aux[0], sb1 = ctx->aux[1], sb2 = ctx->aux[2], sc = ctx->aux[3];
@@ -336,8 +363,8 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1,
   // The G1 sums stay in XYZZ coordinates: only pi_A (beside its scaling) and pi_C are converted.
   // C hands its buckets to H (xH is then the sum of both)
   MsmConfig cfg_a, cfg_b1, share_c, share_h;
-  cfg_a.xyzz_out = xA;
-  cfg_b1.xyzz_out = xB1;
+  if (!P.scaled) cfg_a.xyzz_out = xA;
+  cfg_b1.xyzz_out = P.scaled ? rB1 : xB1;
   share_h.xyzz_out = xH;
   if (!P.share_ch) share_c.xyzz_out = xC;
   if (P.share_ch) {
@@ -346,18 +373,28 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1,
     share_h.bucket_ready = ctx->aux_ev[7];
   }
   ok = (e = run_msm(false, wA, pk->a_ext, pk->fa, nv + 2, outA, P.ms_a, P.bytes_a, sa, &cfg_a)) == cudaSuccess &&
-       (e = run_msm(false, wB, pk->b1_ext, pk->fb1, nv + 2, outB1, P.ms_b1, P.bytes_b1, sb1, &cfg_b1)) == cudaSuccess &&
+       (e = run_msm(false, P.scaled ? at(P.wR) : wB, pk->b1_ext, pk->fb1, nv + 2, outB1, P.ms_b1, P.bytes_b1, sb1, &cfg_b1)) == cudaSuccess &&
        (e = run_msm(true, wB, pk->b2_ext, pk->fb2, nv + 2, outB2, P.ms_b2, P.bytes_b2, sb2)) == cudaSuccess &&
        (e = run_msm(false, wA + (size_t)np1 * 8, pk->c + (size_t)np1 * 16, pk->fc, nv - np1, outC, P.ms_c, P.bytes_c,
                     sc, &share_c)) == cudaSuccess;
   if (!ok) { *where = "prove witness MSMs"; return e; }
   if (P.share_ch && (e = cudaEventRecord(ctx->aux_ev[7], sc)) != cudaSuccess) { *where = "prove C buckets"; return e; }
-  {
+  if (P.scaled) {
+    MsmConfig cfg_s;
+    cfg_s.xyzz_out = sA;
+    cudaStreamWaitEvent(ctx->aux_s, ev_w, 0);
+    if ((e = run_msm(false, at(P.wS), pk->a_ext, pk->fa, nv + 2, outA, P.ms_s, P.bytes_a, ctx->aux_s, &cfg_s)) !=
+        cudaSuccess) {
+      *where = "prove scaled MSM";
+      return e;
+    }
+    cudaEventRecord(ctx->aux_ev[9], ctx->aux_s);
+  } else {
     const GlvSplit* gsp = reinterpret_cast<const GlvSplit*>(rs + 32);
     k_scale_point_glv<<<1, kScaleThreads, 0, sa>>>(xA, gsp, sA, outA);             // s * pi_A
     k_scale_point_glv<<<1, kScaleThreads, 0, sb1>>>(xB1, gsp + 1, rB1, nullptr);  // r * pi_B1
+    note_launch(2);
   }
-  note_launch(2);
   // QAP evaluation, H step and H MSM on their own stream
   cudaStream_t sh = ctx->aux_h;
   cudaStreamWaitEvent(sh, ev_w, 0);
@@ -378,6 +415,7 @@ cudaError_t prove_body(cs_ctx* ctx, cs_pk* pk, const ProvePlan& P, Domain* dom1,
     cudaEventRecord(ctx->aux_ev[1 + i], ctx->aux[i]);
     cudaStreamWaitEvent(sh, ctx->aux_ev[1 + i], 0);
   }
+  if (P.scaled) cudaStreamWaitEvent(sh, ctx->aux_ev[9], 0);
   k_final_c<<<1, 32, 0, sh>>>(xH, P.share_ch ? nullptr : xC, sA, rB1, piC);
   note_launch();
   cudaEventRecord(ctx->aux_ev[3], ctx->aux[2]);  // B2 done

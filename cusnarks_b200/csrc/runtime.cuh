@@ -95,7 +95,8 @@ struct cs_ctx {
   // auxiliary streams / events for fork-join pipelines (prove), created on first use
   cudaStream_t aux[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaStream_t aux_h = nullptr;  // QAP -> H step -> H MSM chain of a proof
-  static constexpr int kAuxEvents = 9;
+  cudaStream_t aux_s = nullptr;  // s pi_A of a small proof as an MSM of its own
+  static constexpr int kAuxEvents = 10;
   cudaEvent_t aux_ev[kAuxEvents] = {nullptr};
   bool aux_ready = false;
   // Proof launch sequences captured as CUDA graphs (prove.cu): one per key and scratch arena,
