@@ -17,17 +17,18 @@
 //   4. accumulate: buckets are summed with mixed XYZZ + affine additions.  Buckets are
 //                split into tasks of at most TASK points; tasks run longest first so
 //                warps see similar trip counts.  Partial sums of split buckets are added
-//                back together by a second pass.
-//   5. reduce:   per window, sum_b (b+1) * bucket_b by hierarchical running sums over
-//                segments of 8 buckets (level k leaves sum_i i*y_i with weight 8^k and
-//                the segment total for the next level).
-//   6. finish:   level results are combined with 3-bit Horner steps, windows with c-bit
+//                back together in two passes.
+//   5. reduce:   per window, sum_b (b+1) * bucket_b: levels of 8 buckets per thread by running
+//                sums while there are many (level k leaves sum_i i*y_i with weight 8^k and the
+//                segment total for the next level), then a binary tree that yields the sum of
+//                the values per bit of their index.
+//   6. finish:   the bits' sums are combined by Horner steps, then the windows by c-bit
 //                Horner steps, and the result is converted to affine.
 //
 // Fixed-base variant, for bases that stay resident (a proving key): a table
 // T[j*N + i] = 2^(c j) P_i of W*N affine points is built once, every digit of every
 // scalar goes into ONE set of 2^(c-1) buckets, and steps 5-6 reduce a single window
-// (more 8-bucket levels, no window Horner).  With the per-window tail gone a wider
+// (no window Horner).  With the per-window tail gone a wider
 // window (c ~ 20 at N = 2^20: 13 instead of 16 windows) also cuts the accumulation.
 #pragma once
 #include <cuda_runtime.h>

@@ -11,9 +11,8 @@
 //     instance, and one persistent k_accumulate over the union of tasks, longest first --
 //     the work is split by bucket size, not by instance, so a 2^10 instance next to a 2^20
 //     one costs its share and no launch;
-//   * reduction per window group (instances with equal c are contiguous: one level chain and
-//     one k_window_sum launch per distinct c), and k_bfinish: one warp per instance for the
-//     window Horner and the affine result.
+//   * reduction of all window groups' trees together (instances with equal c are contiguous),
+//     and k_bfinish: one warp per instance for the window Horner and the affine result.
 // Fixed-base instances (resident tables T[j n + i] = 2^(c j) P_i, the proof's MSMs) put every
 // digit into one bucket set and need no window Horner.
 // The sequence contains no allocation and no host synchronisation, so it can be captured in a
@@ -181,7 +180,7 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Latency form (one quad per task) when the tasks fill the quads at most four times over:
+  // Latency form (one group of lanes per task) when the tasks fill the groups at most four times over:
   // four proofs of 2^12 constraints 2.96 -> 2.62 ms a batch; at eight or sixteen times over the
   // thread form wins (sixteen proofs of 2^12: 4.03 vs 4.76 ms).
   const uint64_t resident_threads = (uint64_t)accumulate_grid<F>(dev, sms) * 128;

@@ -1168,10 +1168,15 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // threads the accumulation keeps resident: an MSM whose tasks (at the shortest length) fit
-  // four times over runs in latency form (one quad per task, shortest tasks)
+  // Threads the accumulation keeps resident: an MSM whose tasks (at the shortest length) fit
+  // several times over runs in latency form (one group of lanes per task, shortest tasks).  A group
+  // spends 16 lane products on a G1 addition where a thread spends 10 (64 and about 27 over G2), so
+  // the line lies where the idle lanes run out (us at 4 / 8 / 16 times: G2 fixed-base 8000 terms
+  // 522 / 454 / 455, generic G2 1000 terms 887 / 887 / 924, generic G1 4000 terms 415 / 427, proof
+  // of 2^12 561 / 561 / 531, of 2^13 873 / 759).
   const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
-  const bool latency_mode = rounds_req == 0 && ((uint64_t)nb + (uint64_t)n * W / kMinTask + 1) * 4 <= resident;
+  constexpr uint64_t kRoom = (EC2 ? 8 : 4) * (FIXED ? 2 : 1);
+  const bool latency_mode = rounds_req == 0 && ((uint64_t)nb + (uint64_t)n * W / kMinTask + 1) * kRoom <= resident;
   // Automatic tile: about one task per resident thread, so a mid-size MSM (too many tasks for
   // the latency form, too few to fill the GPU at 64 entries a task) still keeps every thread
   // busy; 64 entries at most, or 96 where buckets average 48 or more (a GLV-split 2^20 MSM
