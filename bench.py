@@ -77,10 +77,10 @@ PRODUCTS_PER_MONT = 136
 MONT_PER_MADD = 11     # mixed addition, 7M + 4S (the canonical count of the MSM cost model)
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_accumulate launch of
 # the 2^20-term fixed-base G1 MSM (window 20), from an ncu capture of that launch
-ACC_TRAFFIC_BYTES = 1_747_153_664 + 68_581_376
+ACC_TRAFFIC_BYTES = 1_759_405_312 + 71_104_512
 # smsp__issue_active (fraction of cycles issuing) and the busiest pipes of the same capture:
 # the counter view of the roofline fraction below, whose peak is a builder-measured rate
-ACC_NCU = {"issue_active": 0.593, "pipe_alu": 0.535, "pipe_fp64": 0.485}
+ACC_NCU = {"issue_active": 0.343, "pipe_fmaheavy": 0.835, "pipe_alu": 0.245}
 L2_BYTES = 126 * 1024 * 1024
 LOG_M = 20
 R_INT, S_INT = 0x1234567890abcdef, 0xfedcba0987654321
@@ -622,7 +622,7 @@ def run_ours(args, world, rank, local):
         "served_vs_plain": round(e2e_val * plain_ms / 1e3, 2),
         "g1_msm_2^20_ms": round(statistics.median(msm_ms), 3),
         "g1_fixed_msm_2^20_ms": round(statistics.median(fixed_ms), 3),
-        "roofline": {"bound": "int issue (ALU column sums + FP64 split products)",
+        "roofline": {"bound": "integer multiply pipe (32x32->64 products of the Montgomery products)",
                      "kernel": "k_accumulate+k_combine (bucket accumulation of the proof's fixed-base G1 MSMs)",
                      "achieved": round(achieved / 1e12, 4), "peak": round(peak_wide / 1e12, 4),
                      "unit": "T wide products/s", "frac": round(achieved / peak_wide, 4),
@@ -631,9 +631,8 @@ def run_ours(args, world, rank, local):
                      "window": window,
                      "basis": "2^20-term fixed-base G1 MSM as in the proof: N*(254/c+1) bucket entries x 11 Montgomery products x 136 32x32->64 "
                               "products / kernel ms (CUDA events around the kernels); peak = live "
-                              "mad.wide.u32 rate (cs_bench_pipe mode 3), the ceiling of a 32-bit CIOS "
-                              "product (this kernel computes products in radix 2^52 on the FP64 pipe); "
-                              "traffic = ncu DRAM bytes per launch"},
+                              "mad.wide.u32 rate (cs_bench_pipe mode 3), the pipe that the kernel's "
+                              "products run on; traffic = ncu DRAM bytes per launch"},
         "e2e": {"value": round(e2e_val, 3), "unit": UNIT, "ms": round(e2e_ms, 3),
                 "h2d_bytes_per_step": wl.h2d_bytes, "d2h_bytes_per_step": wl.d2h_bytes,
                 "basis": f"C-ABI prove server ({args.slots} slots), {len(jobs)} requests submitted at once, "

@@ -1024,19 +1024,16 @@ inline Layout make_layout(uint32_t n, int c, int xyzz_bytes, uint32_t task_len, 
 
 // Batch-affine rounds before the XYZZ accumulation (the expected bucket size is N W /
 // buckets; a round needs about 8 points per bucket to pay).  Measured at 2^20: G1 is
-// fastest without rounds (its XYZZ addition costs 10 products of 136 wide multiplies and
-// already outruns the gather-bound affine round), G2 with two (Fq2 products are 3 Fq
-// products, so the 6-vs-10 product saving outweighs the extra traffic).
+// fastest without rounds (its XYZZ addition, 10 products, outruns the affine round, which
+// waits on its gathers), G2 with two (Fq2 products are 3 Fq products, so the 6-vs-10 product
+// saving outweighs the extra traffic).
 inline int auto_affine_rounds_rt(bool ec2, uint32_t n, int W, size_t nb) {
   // a round runs kAffK pairs per thread in sequence around one inversion: it needs enough
   // pairs (>= 2^22, i.e. N W >= 2^23 entries) to fill the GPU, or its chain sets the latency
   // (2 rounds cost 2.5 ms in a 2^12-term G2 MSM)
   if ((uint64_t)n * W < (1ull << 23)) return 0;
-  // G1 rounds measured slower, alone and inside proofs (2^20 proof 29.1 -> 30.2 ms with one
-  // round, 30.7 ms with two; with the FP64-pipe products 26.5 -> 29.1 ms with one round, the
-  // 2^20 fixed-base MSM 4.28 -> 5.20 ms): its mixed addition is cheap enough that the extra
-  // passes lose.  L2 prefetching the round's gathers a few slots ahead did not help either
-  // (G2 fixed-base 13.10 ms without, 13.27 / 13.31 / 13.40 ms 2 / 4 / 8 slots ahead).
+  // G1: the 2^20 fixed-base MSM takes 3.03 ms without rounds, 3.50 with one, 3.72 with two.
+  // (L2 prefetching the round's gathers a few slots ahead did not help G2 either.)
   const int cap = ec2 ? 2 : 0;
   const double avg = (double)n * W / (double)nb;
   int r = 0;
