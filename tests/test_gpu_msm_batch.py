@@ -133,3 +133,34 @@ def test_batch_config4_sizes_against_oracle(ctx, oracle, ec2):
             assert np.array_equal(got, oracle.msm(ins[q][0][:n], p, ec2=1 if ec2 else 0)), (q, n)
     finally:
         batch.close()
+
+
+@pytest.mark.parametrize("ec2", [False, True])
+def test_batch_equal_and_opposite_points(ctx, oracle, ec2):
+    """Few instances (groups of lanes add up the buckets) of one point each: every addition meets
+    an equal or an opposite point, in the k1 and the k2 halves of G1's split scalars alike."""
+    import torch
+    from oracle.oracle import R, ints_to_limbs
+    lam = 4407920970296243842393367215006156084916469457145843978461  # phi's eigenvalue: k2 = +-1, k1 small
+    assert (lam * lam + lam + 1) % R == 0
+    n = 64
+    runs = [[1] * n, [R - 1, 1] * (n // 2), [lam, R - lam, 2, R - 2] * (n // 4), list(range(1, n + 1))]
+    jobs, keep = [], []
+    for q, ks in enumerate(runs):
+        s = ints_to_limbs(ks)
+        one = _points(ctx, 1, ec2, 700 + q)
+        dp = one.expand(n, -1).contiguous()
+        ds = torch.from_numpy(s.view(np.int32)).cuda()
+        do = torch.zeros(32 if ec2 else 16, dtype=torch.int32, device="cuda")
+        keep.append((s, ds, dp, do))
+        jobs.append((ds.data_ptr(), dp.data_ptr(), n, do.data_ptr()))
+    torch.cuda.synchronize()
+    batch = ctx.msm_batch(jobs, ec2=ec2)
+    try:
+        batch.run(graph=False)
+        ctx.sync()
+        for q, (s, _, dp, do) in enumerate(keep):
+            want = oracle.msm(s, dp.cpu().numpy().view(np.uint32), ec2=1 if ec2 else 0)
+            assert np.array_equal(do.cpu().numpy().view(np.uint32), want), q
+    finally:
+        batch.close()
