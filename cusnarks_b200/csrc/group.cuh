@@ -128,7 +128,10 @@ struct Group {
     }
     // level 4: S1 PPP, R (Q - X3), ZZZ3 = Z3 PPP, with X3 = RR - PPP - 2 Q
     const Fq s1 = val(j == 0 ? 0 : 1, j == 0 ? 2 : 3, a);
-    if (__any_sync(0xffffffffu, same) && same && l == 0) group_add_slow<F>(p, q, q + 16 * C, false, false, scr);
+    if (__any_sync(0xffffffffu, same)) {
+      __syncwarp();  // a vote orders no memory accesses: s1 has been read before level 1 is written over
+      if (same && l == 0) group_add_slow<F>(p, q, q + 16 * C, false, false, scr);
+    }
     finish(dst, p, inf1, inf2, same, live, pr, s1, q, q + 16 * C, false, false);
   }
 
@@ -153,8 +156,8 @@ struct Group {
     put(2, select_fq(j == 0, pr, lds_fq(at(p, j == 1 ? 0 : 2, a))), val(1, 0, b));
     // level 4: Y1 PPP, R (Q - X3), ZZZ1 PPP
     const Fq s1 = lds_fq(at(p, j == 0 ? 1 : 3, a));
-    if (__any_sync(0xffffffffu, same) && same && l == 0)
-      group_add_slow<F>(p, qx, qy, true, neg, scr);  // level 1 of the scratch is free again
+    // level 1 of the scratch was last read before level 2's barriers
+    if (__any_sync(0xffffffffu, same) && same && l == 0) group_add_slow<F>(p, qx, qy, true, neg, scr);
     finish(dst, p, inf1, false, same, live, pr, s1, qx, qy, true, neg);
   }
 
