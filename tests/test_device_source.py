@@ -1,0 +1,47 @@
+"""Rules of the inline PTX, checked on the source text (no GPU needed): the compiler may move an asm
+statement that is not volatile, and one between the instructions of a carry chain would change the
+flag."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cusnarks_b200", "csrc")
+FILES = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")))
+STRING = re.compile(r'"((?:[^"\\]|\\.)*)"')
+
+
+def _statements(path):
+    """(line, volatile, instructions) of each asm statement."""
+    text = open(path).read().replace("\\\n", "  ")
+    for m in re.finditer(r"\basm\b\s*(volatile)?\s*\(", text):
+        depth, i, quoted = 1, m.end(), False
+        while depth:
+            c = text[i]
+            if c == '"' and text[i - 1] != "\\":
+                quoted = not quoted
+            elif not quoted:
+                depth += (c == "(") - (c == ")")
+            i += 1
+        body = text[m.end():i - 1]
+        template, rest = "", body.lstrip()
+        while rest.startswith('"'):
+            s = STRING.match(rest)
+            template += s.group(1)
+            rest = rest[s.end():].lstrip()
+        template = template.replace("\\n", " ").replace("\\t", " ").strip("{} ")
+        ins = [x.strip() for x in template.split(";") if x.strip(" {}")]
+        yield text.count("\n", 0, m.start()) + 1, bool(m.group(1)), ins
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_statements_that_touch_the_carry_flag_are_volatile(name):
+    for line, volatile, ins in _statements(os.path.join(CSRC, name)):
+        ops = [x.split()[0].split(".") for x in ins]
+        flag = any("cc" in op or op[0] in ("addc", "subc", "madc") for op in ops)
+        assert volatile or not flag, f"{name}:{line}"
+
+
+def test_statements_are_found():
+    n = sum(len(list(_statements(os.path.join(CSRC, f)))) for f in FILES)
+    assert n >= 10
