@@ -45,6 +45,8 @@ struct ModR {  // scalar field r (the reference's MOD_FIELD, pidx 1)
 // order.  So every statement that writes or reads the flag is volatile, the rows of products below
 // too: one that was not could be placed between the instructions of a chain.  (Each chain as one
 // statement, none volatile: 0.2-1 % slower, H step on the coset 2^15 84.5 against 85.3 us.)
+// An output that a statement writes before it has read its last input is early-clobbered (&):
+// otherwise an input of the same value as another operand may be given the output's register.
 #define ADD_CC(d, a, b)     asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 #define ADDC_CC(d, a, b)    asm volatile("addc.cc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 #define ADDC(d, a, b)       asm volatile("addc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
@@ -89,8 +91,8 @@ CSB_DEV void eo_mad(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a)[8], 
       "madc.lo.cc.u32 %4, %20, %24, %4;\n\tmadc.hi.cc.u32 %5, %20, %24, %5;\n\t"
       "madc.lo.cc.u32 %6, %22, %24, %6;\n\tmadc.hi.cc.u32 %7, %22, %24, %7;\n\t"
       "addc.u32 %15, %15, 0;\n\t}"
-      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(o[0]),
-        "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7])
+      : "+&r"(e[0]), "+&r"(e[1]), "+&r"(e[2]), "+&r"(e[3]), "+&r"(e[4]), "+&r"(e[5]), "+&r"(e[6]), "+&r"(e[7]), "+&r"(o[0]),
+        "+&r"(o[1]), "+&r"(o[2]), "+&r"(o[3]), "+&r"(o[4]), "+&r"(o[5]), "+&r"(o[6]), "+&r"(o[7])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b));
 }
 // (e, o) <- ((e, o) >> 32) + a * b, for e[0] = 0.  The left-over limb e[1] goes into the new
@@ -109,7 +111,7 @@ CSB_DEV void eo_shift_mad(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a
       "madc.lo.cc.u32 %4, %27, %31, %4;\n\tmadc.hi.cc.u32 %5, %27, %31, %5;\n\t"
       "madc.lo.cc.u32 %6, %29, %31, %6;\n\tmadc.hi.cc.u32 %7, %29, %31, %7;\n\t"
       "addc.u32 %15, %15, 0;\n\t}"
-      : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7]), "=&r"(n0),
+      : "+&r"(o[0]), "+&r"(o[1]), "+&r"(o[2]), "+&r"(o[3]), "+&r"(o[4]), "+&r"(o[5]), "+&r"(o[6]), "+&r"(o[7]), "=&r"(n0),
         "=&r"(n1), "=&r"(n2), "=&r"(n3), "=&r"(n4), "=&r"(n5), "=&r"(n6), "=&r"(n7)
       : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(a[0]), "r"(a[1]), "r"(a[2]),
         "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b));
@@ -129,18 +131,18 @@ CSB_DEV void pair_chain(uint32_t* t, uint32_t& c, const uint32_t* x, uint32_t b)
   if constexpr (N == 1)
     asm volatile(
         "mad.lo.cc.u32 %0, %3, %4, %0;\n\tmadc.hi.cc.u32 %1, %3, %4, %1;\n\taddc.u32 %2, %2, 0;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(c) : "r"(x[0]), "r"(b));
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(c) : "r"(x[0]), "r"(b));
   if constexpr (N == 2)
     asm volatile(
         "mad.lo.cc.u32 %0, %5, %7, %0;\n\tmadc.hi.cc.u32 %1, %5, %7, %1;\n\t"
         "madc.lo.cc.u32 %2, %6, %7, %2;\n\tmadc.hi.cc.u32 %3, %6, %7, %3;\n\taddc.u32 %4, %4, 0;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(c) : "r"(x[0]), "r"(x[2]), "r"(b));
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(c) : "r"(x[0]), "r"(x[2]), "r"(b));
   if constexpr (N == 3)
     asm volatile(
         "mad.lo.cc.u32 %0, %7, %10, %0;\n\tmadc.hi.cc.u32 %1, %7, %10, %1;\n\t"
         "madc.lo.cc.u32 %2, %8, %10, %2;\n\tmadc.hi.cc.u32 %3, %8, %10, %3;\n\t"
         "madc.lo.cc.u32 %4, %9, %10, %4;\n\tmadc.hi.cc.u32 %5, %9, %10, %5;\n\taddc.u32 %6, %6, 0;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(c)
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(c)
         : "r"(x[0]), "r"(x[2]), "r"(x[4]), "r"(b));
   if constexpr (N == 4)
     asm volatile(
@@ -148,7 +150,7 @@ CSB_DEV void pair_chain(uint32_t* t, uint32_t& c, const uint32_t* x, uint32_t b)
         "madc.lo.cc.u32 %2, %10, %13, %2;\n\tmadc.hi.cc.u32 %3, %10, %13, %3;\n\t"
         "madc.lo.cc.u32 %4, %11, %13, %4;\n\tmadc.hi.cc.u32 %5, %11, %13, %5;\n\t"
         "madc.lo.cc.u32 %6, %12, %13, %6;\n\tmadc.hi.cc.u32 %7, %12, %13, %7;\n\taddc.u32 %8, %8, 0;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(c)
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(t[6]), "+&r"(t[7]), "+&r"(c)
         : "r"(x[0]), "r"(x[2]), "r"(x[4]), "r"(x[6]), "r"(b));
 }
 // lo, hi = a * b
@@ -215,8 +217,8 @@ CSB_DEV void sqr_wide(uint32_t (&t)[16], const uint32_t (&a)[8]) {
       "madc.lo.cc.u32 %10, %21, %21, %10;\n\tmadc.hi.cc.u32 %11, %21, %21, %11;\n\t"
       "madc.lo.cc.u32 %12, %22, %22, %12;\n\tmadc.hi.cc.u32 %13, %22, %22, %13;\n\t"
       "madc.lo.cc.u32 %14, %23, %23, %14;\n\tmadc.hi.u32 %15, %23, %23, %15;"
-      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]),
-        "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
+      : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(t[6]), "+&r"(t[7]), "+&r"(t[8]),
+        "+&r"(t[9]), "+&r"(t[10]), "+&r"(t[11]), "+&r"(t[12]), "+&r"(t[13]), "+&r"(t[14]), "+&r"(t[15])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
 }
 // (e, o) <- ((e, o) >> 32) + p * m with m = -(column 0) / p mod 2^32, for e[0] = 0: one
@@ -232,7 +234,7 @@ CSB_DEV void eo_shift_reduce(uint32_t (&e)[8], uint32_t (&o)[8]) {
       "madc.lo.cc.u32 %3, %19, %9, %13;\n\tmadc.hi.cc.u32 %4, %19, %9, %14;\n\t"
       "madc.lo.cc.u32 %5, %20, %9, %15;\n\tmadc.hi.cc.u32 %6, %20, %9, %16;\n\t"
       "madc.lo.cc.u32 %7, %21, %9, 0;\n\tmadc.hi.u32 %8, %21, %9, 0;"
-      : "+r"(o[0]), "=&r"(n0), "=&r"(n1), "=&r"(n2), "=&r"(n3), "=&r"(n4), "=&r"(n5), "=&r"(n6), "=&r"(n7), "=&r"(m)
+      : "+&r"(o[0]), "=&r"(n0), "=&r"(n1), "=&r"(n2), "=&r"(n3), "=&r"(n4), "=&r"(n5), "=&r"(n6), "=&r"(n7), "=&r"(m)
       : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(M::NP0), "r"(P[1]), "r"(P[3]),
         "r"(P[5]), "r"(P[7]));
 #pragma unroll

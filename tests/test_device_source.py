@@ -1,6 +1,6 @@
 """Rules of the inline PTX, checked on the source text (no GPU needed): the compiler may move an asm
 statement that is not volatile, and one between the instructions of a carry chain would change the
-flag."""
+flag; and it may give an input the register of an output that is not marked early-clobbered."""
 import os
 import re
 
@@ -12,7 +12,7 @@ STRING = re.compile(r'"((?:[^"\\]|\\.)*)"')
 
 
 def _statements(path):
-    """(line, volatile, instructions) of each asm statement."""
+    """(line, volatile, instructions, constraints of the outputs) of each asm statement."""
     text = open(path).read().replace("\\\n", "  ")
     for m in re.finditer(r"\basm\b\s*(volatile)?\s*\(", text):
         depth, i, quoted = 1, m.end(), False
@@ -31,15 +31,26 @@ def _statements(path):
             rest = rest[s.end():].lstrip()
         template = template.replace("\\n", " ").replace("\\t", " ").strip("{} ")
         ins = [x.strip() for x in template.split(";") if x.strip(" {}")]
-        yield text.count("\n", 0, m.start()) + 1, bool(m.group(1)), ins
+        outs = rest[1:].split(":")[0] if rest.startswith(":") else ""
+        yield text.count("\n", 0, m.start()) + 1, bool(m.group(1)), ins, STRING.findall(outs)
 
 
 @pytest.mark.parametrize("name", FILES)
 def test_statements_that_touch_the_carry_flag_are_volatile(name):
-    for line, volatile, ins in _statements(os.path.join(CSRC, name)):
+    for line, volatile, ins, _ in _statements(os.path.join(CSRC, name)):
         ops = [x.split()[0].split(".") for x in ins]
         flag = any("cc" in op or op[0] in ("addc", "subc", "madc") for op in ops)
         assert volatile or not flag, f"{name}:{line}"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_outputs_written_before_the_last_input_are_early_clobbered(name):
+    for line, _, ins, outs in _statements(os.path.join(CSRC, name)):
+        args = [[int(k) for k in re.findall(r"%(\d+)", x)] for x in ins]
+        last_input = max([i for i, a in enumerate(args) if any(k >= len(outs) for k in a)], default=-1)
+        for k, constraint in enumerate(outs):
+            written = min(i for i, a in enumerate(args) if a and a[0] == k)
+            assert written >= last_input or "&" in constraint, f"{name}:{line}: operand {k}"
 
 
 def test_statements_are_found():
