@@ -101,79 +101,91 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
   b->order.resize(njobs);
   std::iota(b->order.begin(), b->order.end(), 0u);
   std::stable_sort(b->order.begin(), b->order.end(), [&](uint32_t x, uint32_t y) { return win[x] < win[y]; });
-  uint64_t terms = 0, buckets = 0, entries = 0, windows = 0;
-  uint64_t lv = 0, lv2 = 0;
-  bool any_glv = false;
-  for (uint32_t k = 0; k < njobs; k++) {
-    const BatchSpec& j = jobs[b->order[k]];
-    const int c = win[b->order[k]];
-    // generic G1 instances split their scalars as single MSMs do: half the bucket sets and half
-    // the Horner chain (24 instances of 2^10..2^16 terms: 2.85 -> 2.45 ms)
-    const bool glv = !ec2 && !j.fixed && j.n < (1u << 30);
-    const uint32_t W = glv ? (128 + c - 1) / c : 254 / c + 1;
-    const uint32_t sets = j.fixed ? 1u : W;
-    BatchJob bj{};
-    bj.scalars = j.scalars;
-    bj.points = j.points;
-    bj.out = j.out;
-    bj.n = j.n;
-    bj.c = (uint32_t)c;
-    bj.W = W;
-    bj.fixed = j.fixed ? 1u : 0u;
-    bj.sets = sets;
-    bj.glv = glv ? 1u : 0u;
-    bj.term0 = (uint32_t)terms;
-    bj.bucket0 = (uint32_t)buckets;
-    bj.window0 = (uint32_t)windows;
-    if (b->groups.empty() || b->groups.back().c != c)
-      b->groups.push_back(BatchGroup{c, (uint32_t)buckets, 0u, (uint32_t)windows});
-    b->groups.back().windows += sets;
-    terms += j.n;
-    buckets += (uint64_t)sets << (c - 1);
-    entries += (uint64_t)j.n * W * (glv ? 2 : 1);
-    any_glv |= glv;
-    windows += sets;
-    b->jobs.push_back(bj);
+  // Generic G1 instances split their scalars as single MSMs do: half the bucket sets and half the
+  // Horner chain (24 instances of 2^10..2^16 terms: 2.85 -> 2.45 ms).  A split term makes
+  // 2 ceil(128 / c) entries instead of 254 / c + 1, up to a thirteenth more, and takes 64 bytes
+  // of scratch: a batch that only fits without the split, in entries or in memory, goes without.
+  for (bool split = !ec2;; split = false) {
+    b->jobs.clear();
+    b->groups.clear();
+    uint64_t terms = 0, buckets = 0, entries = 0, windows = 0;
+    uint64_t lv = 0, lv2 = 0;
+    bool any_glv = false;
+    for (uint32_t k = 0; k < njobs; k++) {
+      const BatchSpec& j = jobs[b->order[k]];
+      const int c = win[b->order[k]];
+      const bool glv = split && !j.fixed && j.n < (1u << 30);
+      const uint32_t W = glv ? (128 + c - 1) / c : 254 / c + 1;
+      const uint32_t sets = j.fixed ? 1u : W;
+      BatchJob bj{};
+      bj.scalars = j.scalars;
+      bj.points = j.points;
+      bj.out = j.out;
+      bj.n = j.n;
+      bj.c = (uint32_t)c;
+      bj.W = W;
+      bj.fixed = j.fixed ? 1u : 0u;
+      bj.sets = sets;
+      bj.glv = glv ? 1u : 0u;
+      bj.term0 = (uint32_t)terms;
+      bj.bucket0 = (uint32_t)buckets;
+      bj.window0 = (uint32_t)windows;
+      if (b->groups.empty() || b->groups.back().c != c)
+        b->groups.push_back(BatchGroup{c, (uint32_t)buckets, 0u, (uint32_t)windows});
+      b->groups.back().windows += sets;
+      terms += j.n;
+      buckets += (uint64_t)sets << (c - 1);
+      entries += (uint64_t)j.n * W * (glv ? 2 : 1);
+      any_glv |= glv;
+      windows += sets;
+      b->jobs.push_back(bj);
+    }
+    for (const auto& g : b->groups) {
+      const uint64_t n1 = ((uint64_t)1 << (g.c - 1)) / 8 + 1;
+      lv = std::max(lv, (uint64_t)g.windows * n1);
+      lv2 = std::max(lv2, (uint64_t)g.windows * (n1 / 8 + 1));
+    }
+    if (any_glv && entries >= 0x7fffffffull) continue;
+    if (terms >= 0xffffffffull || buckets >= 0xffffffffull || entries >= 0x7fffffffull)
+      return fail_msg(ctx, CS_ERR_ARG, "cs_msm_batch_create: batch too large (terms x windows must stay below 2^31)");
+    MsmBatch& P = b->plan;
+    P.njobs = njobs;
+    P.terms = (uint32_t)terms;
+    P.nbuckets = (uint32_t)buckets;
+    P.nentries = entries;
+    P.nwindows = (uint32_t)windows;
+    P.glv = any_glv;
+    P.lv_points = lv;
+    P.lv2_points = lv2;
+    P.groups = b->groups.data();
+    P.ngroups = (uint32_t)b->groups.size();
+    int tile = task;
+    if (task <= 0) {
+      // about one task per resident accumulation thread (3 blocks of 128 per SM): a batch of
+      // small instances splits its buckets so the accumulation keeps every thread busy.
+      // Measured per batch of proofs (ms; tile 64 / one task per thread / three): 16 x 2^12
+      // 4.03 / 3.53 / 4.29, 4 x 2^14 - / 3.53 / 3.80, 4 x 2^16 - / 9.04 / 9.26.
+      int sms = 148;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+      const uint64_t per = entries / ((uint64_t)sms * 384);
+      tile = (int)std::min<uint64_t>(64, std::max<uint64_t>(kBatchMinTask, per));
+    }
+    P.task = std::min(64, std::max(kBatchMinTask, tile));
+    cudaError_t e = cudaSuccess;
+    if (njobs) {
+      e = cudaMalloc(&b->d_jobs, sizeof(BatchJob) * njobs);
+      if (e == cudaSuccess)
+        e = cudaMemcpy(b->d_jobs, b->jobs.data(), sizeof(BatchJob) * njobs, cudaMemcpyHostToDevice);
+      P.d_jobs = b->d_jobs;
+      b->work_bytes = msm_batch_workspace_bytes(P, ec2 != 0);
+      if (e == cudaSuccess) e = cudaMalloc(&b->d_work, b->work_bytes);
+    }
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || !any_glv) return fail(ctx, e, "cs_msm_batch_create: device buffers");
+    cudaGetLastError();
+    cudaFree(b->d_jobs);
+    b->d_jobs = nullptr;
   }
-  for (const auto& g : b->groups) {
-    const uint64_t n1 = ((uint64_t)1 << (g.c - 1)) / 8 + 1;
-    lv = std::max(lv, (uint64_t)g.windows * n1);
-    lv2 = std::max(lv2, (uint64_t)g.windows * (n1 / 8 + 1));
-  }
-  if (terms >= 0xffffffffull || buckets >= 0xffffffffull || entries >= 0x7fffffffull)
-    return fail_msg(ctx, CS_ERR_ARG, "cs_msm_batch_create: batch too large (terms x windows must stay below 2^31)");
-  MsmBatch& P = b->plan;
-  P.njobs = njobs;
-  P.terms = (uint32_t)terms;
-  P.nbuckets = (uint32_t)buckets;
-  P.nentries = entries;
-  P.nwindows = (uint32_t)windows;
-  P.glv = any_glv;
-  P.lv_points = lv;
-  P.lv2_points = lv2;
-  P.groups = b->groups.data();
-  P.ngroups = (uint32_t)b->groups.size();
-  if (task <= 0) {
-    // about one task per resident accumulation thread (3 blocks of 128 per SM): a batch of
-    // small instances splits its buckets so the accumulation keeps every thread busy.
-    // Measured per batch of proofs (ms; tile 64 / one task per thread / three): 16 x 2^12
-    // 4.03 / 3.53 / 4.29, 4 x 2^14 - / 3.53 / 3.80, 4 x 2^16 - / 9.04 / 9.26.
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    const uint64_t per = entries / ((uint64_t)sms * 384);
-    task = (int)std::min<uint64_t>(64, std::max<uint64_t>(kBatchMinTask, per));
-  }
-  P.task = std::min(64, std::max(kBatchMinTask, task));
-  cudaError_t e = cudaSuccess;
-  if (njobs) {
-    e = cudaMalloc(&b->d_jobs, sizeof(BatchJob) * njobs);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_jobs, b->jobs.data(), sizeof(BatchJob) * njobs, cudaMemcpyHostToDevice);
-    P.d_jobs = b->d_jobs;
-    b->work_bytes = msm_batch_workspace_bytes(P, ec2 != 0);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_work, b->work_bytes);
-  }
-  if (e != cudaSuccess) return fail(ctx, e, "cs_msm_batch_create: device buffers");
   *out = b.release();
   return CS_OK;
 }

@@ -164,3 +164,21 @@ def test_batch_equal_and_opposite_points(ctx, oracle, ec2):
             assert np.array_equal(do.cpu().numpy().view(np.uint32), want), q
     finally:
         batch.close()
+
+
+def test_batch_at_the_entry_limit(ctx):
+    """Split scalars make 2 ceil(128 / 17) = 16 entries a term where whole ones make 254 / 17 + 1 = 15:
+    a G1 batch whose 15 n entries stay below 2^31 is planned (without the split where 16 n do not), one
+    entry past it is refused.  Plans only: nothing reads the inputs."""
+    import torch
+    from cusnarks_b200 import CsError
+    x = torch.zeros(64, dtype=torch.int32, device="cuda")
+    for n, fits in ((2 ** 31 // 15, True), (2 ** 31 // 15 + 1, False)):
+        jobs = [(x.data_ptr(), x.data_ptr(), n, x.data_ptr(), 17)]
+        if fits:
+            batch = ctx.msm_batch(jobs)
+            assert batch.windows() == [17] and batch.workspace_bytes() >= 4 * 15 * n
+            batch.close()
+        else:
+            with pytest.raises(CsError):
+                ctx.msm_batch(jobs)
