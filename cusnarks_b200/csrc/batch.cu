@@ -155,6 +155,7 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
     P.nentries = entries;
     P.nwindows = (uint32_t)windows;
     P.glv = any_glv;
+    P.fixed = std::all_of(jobs, jobs + njobs, [](const BatchSpec& j) { return j.fixed; });
     P.lv_points = lv;
     P.lv2_points = lv2;
     P.groups = b->groups.data();

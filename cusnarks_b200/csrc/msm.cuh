@@ -71,6 +71,7 @@ struct MsmBatch {
   const BatchGroup* groups = nullptr;  // host array
   uint32_t ngroups = 0;
   bool glv = false;        // some instance is split (its side arrays are sized by terms)
+  bool fixed = true;       // every instance is fixed-base
   int task = 64;           // entries per accumulation task, kBatchMinTask..64 (set by the builder)
 };
 constexpr int kBatchMinTask = 8;

@@ -180,11 +180,16 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Latency form (one group of lanes per task) when the tasks fill the groups at most four times over:
-  // four proofs of 2^12 constraints 2.96 -> 2.62 ms a batch; at eight or sixteen times over the
-  // thread form wins (sixteen proofs of 2^12: 4.03 vs 4.76 ms).
-  const uint64_t resident_threads = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
-  const bool latency_mode = ((uint64_t)nb + b.nentries / task_len + 1) * 4 <= resident_threads * 4;
+  // Latency form (one group of lanes per task) while the resident threads would fit the tasks (an
+  // upper bound: every bucket and every full tile) this many times: 4, or 16 over tables,
+  // where a batch of proofs runs three batches of MSMs side by side.
+  // Measured (us, groups / threads; in brackets how many times the tasks fit): G1 instances of
+  // 1,351 terms together (8.0) 363 / 368, of 2,791 (3.9) 390 / 380; G2 of 1,351 (5.2) 908 / 924, of
+  // 2,791 (2.5) 1004 / 955; two proofs of 2^7 (17-53) 444 / 447, of 2^8 (9-28) 457 / 455, of 2^9
+  // (6-17) 521 / 490, four of 2^10 (1.5-4.6) 736 / 585.
+  const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
+  const uint64_t room = b.fixed ? 16 : 4;
+  const bool latency_mode = ((uint64_t)nb + b.nentries / task_len + 1) * room <= resident;
   if (latency_mode)
     k_accumulate_group<F><<<sms * 8, 128, 0, st>>>(tasks, counters, entries, nullptr, nb, buckets, partials, b.d_jobs,
                                                     phix);
@@ -194,7 +199,6 @@ cudaError_t batch_impl(const MsmBatch& b, void* d_work, size_t work_bytes, cudaS
   k_combine_small<F><<<sms * 4, 128, 0, st>>>(multi, counters, nb, partials, buckets);
   k_combine<F><<<sms * 4, 128, 0, st>>>(multi, counters, partials, buckets);
   note_launch(3);
-  const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
   // reduction: the groups that need levels of eight (and their buffers) one by one, the others'
   // trees together (24 instances of six widths 3098 -> 2850 us, where each width took a chain of
   // three launches)

@@ -190,3 +190,35 @@ def test_prove_batch_matches_cpu(ctx, oracle):
         batch(plain, 2)
     finally:
         plain.close()
+
+
+# the accumulation of the batch's MSMs: groups of lanes in all of them, in G2 and H only, in none
+@pytest.mark.parametrize("log_m,k", [(5, 2), (8, 2), (10, 3)])
+def test_prove_batch_forms_with_repeated_points(ctx, oracle, log_m, k):
+    """Keys whose points are all one point, and witnesses of 0, 1, -1 and a few repeated values:
+    every addition of the accumulation meets equal or opposite points or infinity."""
+    import torch
+    from cusnarks_b200.groth import SyntheticCircuit, setup_pk, pk_to_host, Prover
+    circ = SyntheticCircuit(ctx, log_m, seed=61, n_inputs=8)
+    host = pk_to_host(setup_pk(ctx, circ, seed=62))
+    for name in ("A", "B1", "B2", "C", "hExps"):
+        host[name] = np.repeat(host[name][7:8], len(host[name]), axis=0)
+    rng = np.random.Generator(np.random.PCG64(63))
+    values = ints_to_limbs([0, 1, R - 1, 2, R - 2, 5])
+    ws = [np.ascontiguousarray(values[rng.integers(0, len(values), circ.n_vars)]) for _ in range(k)]
+    for w in ws:
+        w[0] = values[1]
+    rs, ss = [1, 0, R - 1][:k], [R - 1, 1, 77][:k]
+    prover = Prover(ctx, host, fixed_base=0)
+    try:
+        dws = [torch.from_numpy(w.view(np.int32)).cuda() for w in ws]
+        dp = torch.zeros((k, 64), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        prover.prove_batch_device([t.data_ptr() for t in dws], [ints_to_limbs([x])[0] for x in rs],
+                                  [ints_to_limbs([x])[0] for x in ss], [dp[i].data_ptr() for i in range(k)])
+        ctx.sync()
+        got = dp.cpu().numpy().view(np.uint32)
+        for i in range(k):
+            assert np.array_equal(got[i], cpu_prove(oracle, host, ws[i], rs[i], ss[i])), i
+    finally:
+        prover.close()
