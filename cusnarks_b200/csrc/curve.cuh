@@ -158,13 +158,6 @@ CSB_DEV XYZZ<F> xyzz_add(const XYZZ<F>& p, const XYZZ<F>& q) {
 template <class F>
 __device__ __noinline__ XYZZ<F> xyzz_add_cold(const XYZZ<F> p, const XYZZ<F> q) { return xyzz_add(p, q); }
 
-template <class F>
-CSB_DEV XYZZ<F> xyzz_neg(const XYZZ<F>& p) {
-  XYZZ<F> r = p;
-  r.Y = p.Y.neg();
-  return r;
-}
-
 // XYZZ -> affine with the reference infinity encoding
 template <class F>
 CSB_DEV Affine<F> xyzz_to_affine(const XYZZ<F>& p) {

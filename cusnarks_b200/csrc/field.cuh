@@ -268,7 +268,6 @@ struct Fp {
     return ((v[0] ^ o.v[0]) | (v[1] ^ o.v[1]) | (v[2] ^ o.v[2]) | (v[3] ^ o.v[3]) |
             (v[4] ^ o.v[4]) | (v[5] ^ o.v[5]) | (v[6] ^ o.v[6]) | (v[7] ^ o.v[7])) == 0;
   }
-  CSB_DEV bool is_one() const { return *this == one(); }
 
   // r = t - p if t >= p else t, for t < 2p (t given in 8 limbs).
   static CSB_DEV void reduce_once(uint32_t (&t)[8]) {
@@ -394,10 +393,7 @@ struct Fp {
 
   // ---- lazily reduced values in [0, 2p) (BN254: 4p < 2^256): products of two such values
   // are below 2p without the final subtraction (1.76 p)
-  static CSB_DEV Fp mul_lazy(const Fp& a, const Fp& b);
-  static CSB_DEV Fp sqr_lazy(const Fp& a);
-  // a b - c d for values < 2p, result < 2p: a b + (2p - c) d is below 2.51 p
-  static CSB_DEV Fp mul_sub_lazy(const Fp& a, const Fp& b, const Fp& c, const Fp& d);
+
   // 2p, limb i
   static CSB_DEV uint32_t p2(int i) {
     const uint32_t P[8] = {M::P0, M::P1, M::P2, M::P3, M::P4, M::P5, M::P6, M::P7};
@@ -519,21 +515,8 @@ __device__ __noinline__ Fp<M> fp_mul_call(Fp<M> a, Fp<M> b) {
 }
 
 template <class M>
-__device__ __noinline__ Fp<M> fp_mul_lazy_call(Fp<M> a, Fp<M> b) {
-  return Fp<M>::mul_raw(a, b);
-}
-
-template <class M>
-__device__ __noinline__ Fp<M> fp_sqr_lazy_call(Fp<M> a) {
-  return Fp<M>::sqr_raw(a);
-}
-template <class M>
 __device__ __noinline__ Fp<M> fp_sqr_call(Fp<M> a) {
   return Fp<M>::sqr_raw(a).canon();
-}
-template <class M>
-__device__ __noinline__ Fp<M> fp_mul2_call(Fp<M> a, Fp<M> b, Fp<M> c, Fp<M> d) {
-  return Fp<M>::mul2_raw(a, b, c, d);
 }
 
 template <class M>
@@ -549,26 +532,10 @@ CSB_DEV Fp<M> Fp<M>::inv() const { return fp_inv_call<M>(*this); }
 // Out of line (CSB_MUL_NOINLINE units) or inlined
 #if defined(CSB_MUL_NOINLINE)
 template <class M>
-CSB_DEV Fp<M> Fp<M>::mul_lazy(const Fp<M>& a, const Fp<M>& b) { return fp_mul_lazy_call<M>(a, b); }
-template <class M>
-CSB_DEV Fp<M> Fp<M>::sqr_lazy(const Fp<M>& a) { return fp_sqr_lazy_call<M>(a); }
-template <class M>
 CSB_DEV Fp<M> Fp<M>::sqr() const { return fp_sqr_call<M>(*this); }
-template <class M>
-CSB_DEV Fp<M> Fp<M>::mul_sub_lazy(const Fp<M>& a, const Fp<M>& b, const Fp<M>& c, const Fp<M>& d) {
-  return reduce_2p(fp_mul2_call<M>(a, b, neg_lazy(c), d));
-}
 #else
 template <class M>
-CSB_DEV Fp<M> Fp<M>::mul_lazy(const Fp<M>& a, const Fp<M>& b) { return mul_raw(a, b); }
-template <class M>
-CSB_DEV Fp<M> Fp<M>::sqr_lazy(const Fp<M>& a) { return sqr_raw(a); }
-template <class M>
 CSB_DEV Fp<M> Fp<M>::sqr() const { return sqr_raw(*this).canon(); }
-template <class M>
-CSB_DEV Fp<M> Fp<M>::mul_sub_lazy(const Fp<M>& a, const Fp<M>& b, const Fp<M>& c, const Fp<M>& d) {
-  return reduce_2p(mul2_raw(a, b, neg_lazy(c), d));
-}
 #endif
 
 // ------------------------------------------------------------ Fq2 = Fq[u]/(u^2+1) ----

@@ -74,13 +74,13 @@ __host__ __device__ inline void modinv(const uint32_t* x, const uint32_t* p, uin
   for (int i = 0; i < 8; i++) { a[i] = x[i]; b[i] = p[i]; u[i] = i == 0; v[i] = 0; }
 #pragma unroll 1
   for (int round = 0; round < 17; round++) {
-    // the window of 64 bits below the longer operand's top bit (the three limbs from its
-    // highest nonzero one down); operands that fit 62 bits are taken whole
-    uint32_t a2 = a[1], a1 = a[0], a0 = 0, b2 = b[1], b1 = b[0], b0 = 0;
+    // the two limbs from the longer operand's highest nonzero one down, of which the top 32 bits
+    // are taken; operands that fit 62 bits are taken whole
+    uint32_t a2 = a[1], a1 = a[0], b2 = b[1], b1 = b[0];
     for (int i = 2; i < 8; i++) {
       const bool nz = (a[i] | b[i]) != 0;
-      a2 = nz ? a[i] : a2; a1 = nz ? a[i - 1] : a1; a0 = nz ? a[i - 2] : a0;
-      b2 = nz ? b[i] : b2; b1 = nz ? b[i - 1] : b1; b0 = nz ? b[i - 2] : b0;
+      a2 = nz ? a[i] : a2; a1 = nz ? a[i - 1] : a1;
+      b2 = nz ? b[i] : b2; b1 = nz ? b[i - 1] : b1;
     }
     const bool big = (a[2] | a[3] | a[4] | a[5] | a[6] | a[7] | b[2] | b[3] | b[4] | b[5] | b[6] | b[7]) != 0;
     const uint32_t top = a2 | b2;
@@ -91,7 +91,7 @@ __host__ __device__ inline void modinv(const uint32_t* x, const uint32_t* p, uin
 #endif
     const bool whole = !big && lz >= 2;
     lz &= 31;
-    // top 32 bits of the window
+    // top 32 bits of the two limbs
     const uint32_t ta = (uint32_t)((((uint64_t)a2 << 32 | a1) << lz) >> 32);
     const uint32_t tb = (uint32_t)((((uint64_t)b2 << 32 | b1) << lz) >> 32);
     uint64_t xa = (uint64_t)ta << 30 | (a[0] & 0x3fffffffu), xb = (uint64_t)tb << 30 | (b[0] & 0x3fffffffu);
