@@ -95,13 +95,14 @@ CSB_DEV Block pass_block(const Pass& a) {
   return b;
 }
 
-// Throughput form (2^22 points 0.89 ms, 1.05 ms with one stage a barrier and values reduced below r
-// after each; bound by the products, 0.68 ms at the GPU's rate): a thread takes four elements through two stages at a time, so a pass
-// crosses shared memory and the barrier (S - 1) / 2 times; the first stages read from and
-// the last write to global memory directly.  An odd S starts with one single stage.
-// BLOCKS resident blocks a SM: three (84 registers) from 2^20 points on, where there are blocks
-// enough to keep them full (2^22 893 against 868 us, H step of 2^20 1372 / 1326), two below (H
-// step of 2^18 342 against 363).
+// Throughput form (2^22 points 0.87 ms, bound by the products: 0.68 ms at the GPU's rate; 1.05 ms
+// with one stage a barrier and values reduced below r after each): a thread takes four elements
+// through two stages at a time, so a pass crosses shared memory and the barrier (S - 1) / 2 times;
+// the first stages read from and the last write to global memory directly.  An odd S starts with
+// one single stage.  BLOCKS resident blocks a SM: three (80 registers) from 2^20 elements in all
+// transforms of the launch on, where there are blocks enough to keep them full, two below (us, two /
+// three: NTT 2^19 117 / 122, 2^20 220 / 215, 2^22 896 / 872; H step of 2^18 346 / 371, of 2^19, two
+// transforms side by side, 669 / 648; on the coset, three of them, 2^18 404 / 402, 2^19 774 / 756).
 template <int BLOCKS>
 __global__ void __launch_bounds__(kThreads, BLOCKS) k_ntt_pass4(const Pass a) {
   extern __shared__ uint4 sm[];
@@ -265,7 +266,8 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
     }
   }
   // one thread per butterfly while that leaves at most kLatencyWarps warps a scheduler
-  const bool latency = ((uint64_t)a.count * a.batch << (L - 1)) <= (uint64_t)sms * 4 * 32 * kLatencyWarps;
+  const uint64_t elements = (uint64_t)a.count * a.batch << L;
+  const bool latency = elements / 2 <= (uint64_t)sms * 4 * 32 * kLatencyWarps;
   uint32_t s0 = 0;
   for (int p = 0; p < np; p++) {
     const uint32_t S = sizes[p];
@@ -286,7 +288,7 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
     q.load = (int)a.load;
     q.canon = last && !a.lazy_out;
     const dim3 grid(1u << (L - S), a.batch, a.count);
-    auto* pass4 = L >= 20 ? k_ntt_pass4<3> : k_ntt_pass4<2>;
+    auto* pass4 = elements >= 1u << 20 ? k_ntt_pass4<3> : k_ntt_pass4<2>;
     if ((32u << S) > 48u * 1024) {  // above the default limit of a block's shared memory
       const cudaError_t e = cudaFuncSetAttribute(latency ? (const void*)k_ntt_pass2 : (const void*)pass4,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 32 << S);

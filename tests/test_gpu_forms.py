@@ -43,7 +43,8 @@ def test_ntt_pass_forms(ctx, oracle, L):
         assert np.array_equal(_host(out), want) and np.array_equal(_host(d), want), direction
 
 
-@pytest.mark.parametrize("L", [1, 2, 3, 8, 9, 10, 15, 16, 17])
+# 18, 19: two and three blocks a SM
+@pytest.mark.parametrize("L", [1, 2, 3, 8, 9, 10, 15, 16, 17, 18, 19])
 def test_hstep_forms(ctx, oracle, L):
     rng = np.random.Generator(np.random.PCG64(400 + L))
     m = 1 << L
