@@ -17,7 +17,10 @@
  * uint32 limbs; pidx 0 = base field q (MOD_GROUP), 1 = scalar field r (MOD_FIELD);
  * points are affine Montgomery, G1 = X|Y (16 words), G2 = X.c0|X.c1|Y.c0|Y.c1 (32 words);
  * infinity is (0, 1_mont) in G1 and (0, 0, 1_mont, 0) in G2; MSM scalars are normal form
- * and may take any 256-bit value.
+ * and may take any 256-bit value.  Points lie on their curve: G1 y^2 = x^3 + 3, G2 its twist.
+ * Nothing checks it, but every G1 multi-exponentiation uses it (all of them, batches, fixed
+ * bases and proofs too, double by the curve equation; generic ones split their scalars by an
+ * endomorphism), so the result for points of another curve is unspecified.
  */
 #ifndef CUSNARKS_B200_H
 #define CUSNARKS_B200_H
@@ -223,7 +226,8 @@ int cs_msm_device(cs_ctx *ctx, int ec2, const uint32_t *d_scalars, const uint32_
 /* Scratch bytes one MSM of n terms needs (window 0 = automatic). */
 size_t cs_msm_workspace_bytes(uint32_t n, int ec2, int window);
 /* Window bits the automatic choice uses for n terms (G1: for the GLV split), and the window
- * count of a full scalar (254 / window + 1: G2, fixed-base tables, batch instances). */
+ * count of a full scalar (254 / window + 1: G2 and fixed-base tables; split G1 scalars take
+ * ceil(128 / window)). */
 int cs_msm_default_window(uint32_t n, int ec2);
 int cs_msm_num_windows(int window);
 
@@ -251,7 +255,9 @@ int cs_msm_fixed_device(cs_ctx *ctx, int ec2, const uint32_t *d_scalars, const u
  * captures the sequence into a CUDA graph on the first run and replays it afterwards (the
  * plan's pointers are baked in: change inputs in place).  task = bucket tile (max entries
  * per accumulation task, 8..64; 0 = by the batch's size: about one task per resident
- * accumulation thread, 8..64).  Each result equals cs_msm_device's. */
+ * accumulation thread, 8..64).  G1 instances split their scalars as cs_msm's do, unless the
+ * batch fits only without (2^31 bucket entries; device memory).  Each result equals
+ * cs_msm_device's. */
 typedef struct {
   const uint32_t *scalars, *points;
   uint32_t *out;
@@ -265,9 +271,9 @@ int cs_msm_batch_run(cs_ctx *ctx, cs_msm_batch *batch, int use_graph);
 void cs_msm_batch_destroy(cs_msm_batch *batch);
 size_t cs_msm_batch_workspace_bytes(const cs_msm_batch *batch);
 int cs_msm_batch_window(const cs_msm_batch *batch, uint32_t job);
-/* Window autotuner for batched MSMs: times the MSM of full scalars (the form a batch instance
- * runs) at each size 2^log_min..2^log_max for windows around the cost-model choice and keeps
- * the fastest per size (per device, process-wide); windows_out (optional) receives them.
+/* Window autotuner for batched MSMs: times the MSM (G1 with split scalars, the form a batch
+ * instance runs) at each size 2^log_min..2^log_max for windows around the cost-model choice and
+ * keeps the fastest per size (per device, process-wide); windows_out (optional) receives them.
  * Synchronous. */
 int cs_msm_autotune(cs_ctx *ctx, int ec2, uint32_t log_min, uint32_t log_max, int *windows_out);
 int cs_msm_tuned_window(cs_ctx *ctx, int ec2, uint32_t n);
