@@ -38,8 +38,8 @@ int pick_window(int dev, int ec2, uint32_t n) {
 }
 
 // Pseudo-random limbs for timing runs (splitmix-style hash); top limb masked below 2^253 so
-// scalars are below r.  Coordinates need not be on the curve: the addition formulas run the
-// same instructions either way.
+// scalars are below r.  Coordinates need not be on the curve where the result is not read: the
+// formulas run the same instructions either way.
 __global__ void k_fill_random(uint32_t* p, size_t elems, uint32_t seed) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= elems) return;
@@ -147,7 +147,7 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
     }
     if (any_glv && entries >= 0x7fffffffull) continue;
     if (terms >= 0xffffffffull || buckets >= 0xffffffffull || entries >= 0x7fffffffull)
-      return fail_msg(ctx, CS_ERR_ARG, "cs_msm_batch_create: batch too large (terms x windows must stay below 2^31)");
+      return fail_msg(ctx, CS_ERR_ARG, "cs_msm_batch_create: batch too large (terms x (254 / window + 1) must stay below 2^31)");
     MsmBatch& P = b->plan;
     P.njobs = njobs;
     P.terms = (uint32_t)terms;
@@ -162,10 +162,11 @@ int batch_build(cs_ctx* ctx, int ec2, const BatchSpec* jobs, uint32_t njobs, int
     P.ngroups = (uint32_t)b->groups.size();
     int tile = task;
     if (task <= 0) {
-      // about one task per resident accumulation thread (3 blocks of 128 per SM): a batch of
-      // small instances splits its buckets so the accumulation keeps every thread busy.
-      // Measured per batch of proofs (ms; tile 64 / one task per thread / three): 16 x 2^12
-      // 4.03 / 3.53 / 4.29, 4 x 2^14 - / 3.53 / 3.80, 4 x 2^16 - / 9.04 / 9.26.
+      // 384 tasks a SM, about one per resident accumulation thread (G2 keeps 384, G1 512): a batch
+      // of small instances splits its buckets so the accumulation keeps every thread busy.
+      // Measured for G1 at 512 / 384 / 256 tasks a SM (us): batches of proofs 16 x 2^12 2311 / 2240 /
+      // 2236, 4 x 2^12 1013 / 1029 / 921, 4 x 2^14 2153 / 2123 / 2107, 4 x 2^16 6170 / 6162 / 6165;
+      // eight instances of 2^11..2^12 terms 629 / 584 / 550, of 2^13..2^14 998 / 972 / 1014.
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
       const uint64_t per = entries / ((uint64_t)sms * 384);

@@ -54,9 +54,11 @@ struct ModR {  // scalar field r (the reference's MOD_FIELD, pidx 1)
 #define SUBC_CC(d, a, b)    asm volatile("subc.cc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 #define SUBC(d, a, b)       asm volatile("subc.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b))
 
-// Montgomery products accumulate in two sets of columns: e holds columns 0..7 as the 64-bit
-// pairs (0,1) (2,3) (4,5) (6,7), o columns 1..8 as (1,2) (3,4) (5,6) (7,8), and the value is
-// e + 2^32 o.  A limb's products with the even limbs of the other operand tile e's pairs and
+// Montgomery products accumulate in two sets of columns, the partial products sorted by the
+// alignment of their limbs (as Emmart, Luitjens, Weems and Woolley do for half-word products,
+// "Optimizing modular multiplication for NVIDIA's Maxwell GPUs", ARITH 2016): e holds columns
+// 0..7 as the 64-bit pairs (0,1) (2,3) (4,5) (6,7), o columns 1..8 as (1,2) (3,4) (5,6) (7,8), and
+// the value is e + 2^32 o.  A limb's products with the even limbs of the other operand tile e's pairs and
 // those with its odd limbs tile o's, so every 32x32->64 product is one multiply-add with
 // carry in and out (a mad.lo.cc / madc.hi.cc pair on one aligned pair issues as one wide
 // multiply-add) and no separate additions fold it in.  Shifting the value down one limb

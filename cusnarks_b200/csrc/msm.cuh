@@ -39,8 +39,7 @@ namespace csb {
 
 // Instance of a batch of MSMs: device pointers, size, window, and its first term, bucket
 // and window in the batch (instances are ordered by window so each window group occupies a
-// contiguous bucket range).
-// A batch instance.  fixed = 0: points holds n points, W bucket sets (one per window).
+// contiguous bucket range).  fixed = 0: points holds n points, W bucket sets (one per window).
 // fixed = 1: points is a fixed-base table T[j n + i] = 2^(c j) P_i of W windows, one bucket set
 // (entries are table indices), no window Horner.  sets: bucket sets (W or 1).  glv: a generic G1
 // instance, its scalars split by the endomorphism as a single MSM's are.
@@ -64,9 +63,9 @@ struct MsmBatch {
   const BatchJob* d_jobs = nullptr;
   uint32_t njobs = 0;
   uint32_t terms = 0;      // sum of n
-  uint32_t nbuckets = 0;   // sum of W * 2^(c-1)
-  uint64_t nentries = 0;   // sum of n * W (upper bound of bucket entries)
-  uint32_t nwindows = 0;   // sum of W
+  uint32_t nbuckets = 0;   // sum of sets * 2^(c-1)
+  uint64_t nentries = 0;   // sum of n * W, 2 n * W of split instances (upper bound of bucket entries)
+  uint32_t nwindows = 0;   // sum of sets
   uint64_t lv_points = 0, lv2_points = 0;  // max over groups of W*(2^(c-1)/8+1), W*(.../64+1)
   const BatchGroup* groups = nullptr;  // host array
   uint32_t ngroups = 0;

@@ -1,5 +1,5 @@
 // msm_batch_g1.cu -- G1 (Fq) instantiation of the batched MSM (msm_batch.cuh).
-// Montgomery products out of line, as in the single MSM (instruction-cache fit).
+// Products of operators are calls, as in the single MSM (msm_g1.cu).
 #define CSB_MUL_NOINLINE
 #include "msm_batch.cuh"
 

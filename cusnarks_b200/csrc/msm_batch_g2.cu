@@ -1,5 +1,5 @@
 // msm_batch_g2.cu -- G2 (Fq2) instantiation of the batched MSM (msm_batch.cuh).
-// Montgomery products out of line, as in the single MSM (instruction-cache fit).
+// Fq2 products are calls, as in the single MSM (msm_g2.cu).
 #define CSB_MUL_NOINLINE
 #include "msm_batch.cuh"
 

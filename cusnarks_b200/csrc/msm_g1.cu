@@ -1,6 +1,7 @@
 // msm_g1.cu -- G1 (Fq) instantiation of the MSM pipeline.
-// Montgomery products out of line: the accumulation loop body (one XYZZ + affine
-// addition, 10 products) then fits the instruction cache; measured faster at 2^20.
+// Products of operators are calls here (the bucket reduction's levels and the table kernels
+// chain dozens of them): the same times as inlined (2^20 terms 3655 us both, fixed-base 3052) and
+// a fraction of the code.  The accumulation and the lane groups inline theirs (Fp::mul_raw).
 #define CSB_MUL_NOINLINE
 #include "msm_impl.cuh"
 

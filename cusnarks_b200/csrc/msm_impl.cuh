@@ -893,7 +893,7 @@ CSB_DEV uint32_t bucket_of_slot(const uint32_t* off, uint32_t nb, uint32_t s) {
 }
 
 // At least 3 blocks a SM asked for: over Fq2 the products take 198 registers uncapped, two
-// blocks (2^20 fixed-base G2 MSM 10.44 ms); at 168 registers, three blocks, 9.05 ms.
+// blocks (2^20 fixed-base G2 MSM 8.50 ms); at 168 registers, three blocks, 7.48 ms.
 template <class F, bool FIRST>
 __global__ void __launch_bounds__(128, 3) k_affine_round(const uint32_t* __restrict__ in_off,
                                                       const uint32_t* __restrict__ out_off, uint32_t nb,
@@ -1165,12 +1165,19 @@ cudaError_t msm_impl(const uint32_t* d_scalars, const uint32_t* d_points, uint32
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Threads the accumulation keeps resident: an MSM whose tasks (at the shortest length) fit
-  // several times over runs in latency form (one group of lanes per task, shortest tasks).  A group
-  // spends 16 lane products on a G1 addition where a thread spends 10 (64 and about 27 over G2), so
-  // the line lies where the idle lanes run out (us at 4 / 8 / 16 times: G2 fixed-base 8000 terms
-  // 522 / 454 / 455, generic G2 1000 terms 887 / 887 / 924, generic G1 4000 terms 415 / 427, proof
-  // of 2^12 561 / 561 / 531, of 2^13 873 / 759).
+  // Threads the accumulation keeps resident: an MSM whose tasks (an upper bound, at 32 entries)
+  // fit kRoom times over runs in latency form (one group of lanes per task, shortest tasks).  A
+  // group spends 16 lane products on a G1 addition where a thread spends 10 (64 and about 27 over
+  // G2), so the line lies where the idle lanes run out: over tables, where tiles rather than buckets
+  // make the tasks, twice as early, because the groups' tiles of 16 are twice as many.  Measured (us,
+  // groups / threads; in brackets how many times the tasks fit):
+  //   generic G2  1,000 terms (11.2) 881 / 910, 2,000 (9.3) 931 / 934, 4,000 (5.1) 1024 / 990
+  //   fixed G2    1,000 (32) 311 / 343, 2,000 (16.6) 363 / 365, 8,000 (6.2) 534 / 455
+  //   generic G1  1,000 (25) 395 / 392, 4,000 (7.6) 430 / 436, 8,000 (4.1) 500 / 467, 12,000 (3.6)
+  //               531 / 507
+  //   fixed G1    1,000 (43) 247 / 233, 4,000 (11.5) 248 / 251, 8,000 (8.3) 297 / 277, 16,000 (3.0)
+  //               322 / 299
+  // (over Fq the two are within 7 % of each other up to the line).
   const uint64_t resident = (uint64_t)accumulate_grid<F>(dev, sms) * 128;
   constexpr uint64_t kRoom = (EC2 ? 8 : 4) * (FIXED ? 2 : 1);
   const bool latency_mode = rounds_req == 0 && ((uint64_t)nb + (uint64_t)n * W / kMinTask + 1) * kRoom <= resident;
