@@ -11,7 +11,7 @@ reference's own CPU library (oracle/_ref), never GPU against GPU:
   fixed-base table and the G1 MSMs the throughput form of the bucket accumulation.
 The CPU builder of the benchmark circuit and key (oracle/synth_cpu.py, which bench.py's
 reference arm uses) is checked against the GPU builder word for word.  A 2^22-constraint proof
-is checked by the pairing equation; proofs of 2^15 and 2^17 constraints and a generic G2 MSM of
+is checked by the pairing equation; proofs of 2^13 to 2^17 constraints and a generic G2 MSM of
 2^15 terms (mid sizes, whose accumulation tasks are sized to the GPU) against the CPU.
 """
 import numpy as np
@@ -191,12 +191,13 @@ def test_prove_2e22_verifies(ctx):
     assert not verify(pk["vk"], proof, bad)
 
 
-@pytest.mark.parametrize("log_m", [15, 17])
+@pytest.mark.parametrize("log_m", [13, 14, 15, 17])
 def test_prove_mid_sizes_match_cpu(ctx, oracle, log_m):
-    """Proofs of 2^15 and 2^17 constraints, where the MSMs are too large for the latency form
-    and too small to fill the GPU at full-length tasks (their accumulation tasks are sized to
-    the GPU): byte for byte the CPU proving sequence (the reference library where built),
-    and the pairing check."""
+    """Proofs of 2^13 constraints, the last whose s pi_A and r pi_B1 are MSMs of scaled scalars,
+    and of 2^14, the first whose are not; of 2^15 and 2^17, where the MSMs are too large for the
+    latency form and too small to fill the GPU at full-length tasks (their accumulation tasks are
+    sized to the GPU): byte for byte the CPU proving sequence (the reference library where
+    built), and the pairing check."""
     from cusnarks_b200.groth import SyntheticCircuit, setup_pk, pk_to_host, Prover
     from oracle.oracle import RefLib
     from oracle.prover import cpu_prove, verify

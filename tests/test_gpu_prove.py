@@ -115,9 +115,9 @@ def test_dropin_mpoly_eval_fixture(golden):
 
 
 def test_prove_graph_replays_match_cpu(ctx, oracle):
-    """The proof's launch sequence is captured as a CUDA graph on the first proof with a key,
-    witness buffer and scratch, then replayed: replays with new r, s and a new witness in the
-    same buffer give the CPU sequence's bytes; rebuilt tables and graphs turned off too."""
+    """The proof's launch sequence is captured as a CUDA graph on the first proof with a key
+    and scratch, then replayed: replays with new r, s and a new witness in the same buffer give
+    the CPU sequence's bytes; rebuilt tables and graphs turned off too."""
     import pytest as _pt
     from cusnarks_b200._lib import CsError
     from cusnarks_b200.groth import SyntheticCircuit, setup_pk, pk_to_host, Prover
@@ -146,6 +146,36 @@ def test_prove_graph_replays_match_cpu(ctx, oracle):
     finally:
         ctx.set_prove_graphs(True)
         prover.close()
+
+
+def test_prove_graph_replays_other_witness_buffers(ctx, oracle):
+    """A replay takes its witness from whatever device buffer the call names: proofs of three
+    buffers, the first again after the others, enqueued one behind the other without waiting."""
+    import torch
+    from cusnarks_b200.groth import SyntheticCircuit, setup_pk, pk_to_host, Prover
+    from oracle.oracle import random_field
+    circ = SyntheticCircuit(ctx, 7, seed=81)
+    pk = setup_pk(ctx, circ, seed=82)
+    host = pk_to_host(pk)
+    rng = np.random.Generator(np.random.PCG64(83))
+    ws = [circ.w] + [random_field(rng, circ.n_vars, 1) for _ in range(2)]
+    for w in ws[1:]:
+        w[0] = ints_to_limbs([1])[0]
+    order = [0, 1, 2, 0, 2, 1]
+    dws = [torch.from_numpy(np.ascontiguousarray(w).view(np.int32)).cuda() for w in ws]
+    dp = torch.zeros((len(order), 64), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    prover = Prover(ctx, pk)
+    try:
+        for i, k in enumerate(order):
+            prover.prove_device(dws[k].data_ptr(), ints_to_limbs([5 + i])[0], ints_to_limbs([R - 3 - i])[0],
+                                dp[i].data_ptr())
+        ctx.sync()
+    finally:
+        prover.close()
+    got = dp.cpu().numpy().view(np.uint32)
+    for i, k in enumerate(order):
+        assert np.array_equal(got[i], cpu_prove(oracle, host, ws[k], 5 + i, R - 3 - i)), i
 
 
 def test_prove_batch_matches_cpu(ctx, oracle):
