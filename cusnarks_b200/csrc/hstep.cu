@@ -467,7 +467,7 @@ int cs_ntt_device(cs_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint32_t l
   cudaError_t e = domain_get(ctx, log_n, &dom);
   if (e != cudaSuccess) return fail(ctx, e, "ntt domain");
   const size_t bytes = ((size_t)32 << log_n);
-  if (d_in == d_out) {
+  if (ntt_overlap(d_in, d_out, log_n)) {
     if ((e = ctx->work.reserve(bytes, ctx->stream)) != cudaSuccess) return fail(ctx, e, "ntt scratch");
   }
   NttArgs t;

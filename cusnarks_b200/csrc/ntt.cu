@@ -258,9 +258,11 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
   plan_passes(L, sizes, &np);
   uint32_t* work = a.out;
   if (np > 1) {
-    bool alias = false;
-    for (uint32_t z = 0; z < a.count; z++) alias |= a.in[z] == a.out + z * a.out_step;
-    if (alias) {
+    // the first pass must not write where other blocks still read
+    bool over = false;
+    for (uint32_t z = 0; z < a.count; z++)
+      for (uint32_t y = 0; y < a.count; y++) over |= ntt_overlap(a.in[z], a.out + y * a.out_step, L);
+    if (over) {
       if (!a.tmp) return cudaErrorInvalidValue;
       work = a.tmp;
     }

@@ -28,9 +28,9 @@ struct NttArgs {
   // addresses): transform z reads in[z] and writes out + z * out_step words
   const uint32_t* in[3] = {nullptr, nullptr, nullptr};
   uint32_t count = 1;
-  uint32_t* out = nullptr;          // natural-order output; may equal in[0] where tmp is given
+  uint32_t* out = nullptr;          // natural-order output; may lie over in[] where tmp is given
   size_t out_step = 0;
-  uint32_t* tmp = nullptr;          // scratch, laid out as out, when out aliases the input
+  uint32_t* tmp = nullptr;          // scratch, laid out as out, when out overlaps the input
   uint32_t log_n = 0;
   const uint32_t* W = nullptr;      // twiddles for direction of this transform
   uint32_t log_tab = 0;             // W is a table for 2^log_tab points
@@ -46,6 +46,11 @@ struct NttArgs {
 };
 
 cudaError_t ntt_run(const NttArgs& a, cudaStream_t st);
+// Whether two arrays of 2^log_n elements overlap.
+inline bool ntt_overlap(const uint32_t* x, const uint32_t* y, uint32_t log_n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y), n = (uintptr_t)32 << log_n;
+  return a < b + n && b < a + n;
+}
 
 // W[j] = root^j for j < count (root: one Montgomery element in device memory).
 cudaError_t ntt_powers(uint32_t* d_out, const uint32_t* d_root, uint32_t count, cudaStream_t st);

@@ -43,6 +43,18 @@ def test_ntt_pass_forms(ctx, oracle, L):
         assert np.array_equal(_host(out), want) and np.array_equal(_host(d), want), direction
 
 
+@pytest.mark.parametrize("L", [8, 9, 11, 12])
+@pytest.mark.parametrize("shift", [-1, 1, 100])
+def test_ntt_output_partly_over_its_input(ctx, oracle, L, shift):
+    rng = np.random.Generator(np.random.PCG64(350 + L))
+    n = 1 << L
+    A = oracle.to_mont(random_field(rng, n, 1), 1)
+    buf = _dev(np.concatenate([np.zeros((100, 8), np.uint32), A, np.zeros((100, 8), np.uint32)]))
+    ctx.ntt_device(buf.data_ptr() + 32 * 100, buf.data_ptr() + 32 * (100 + shift), L, 1)
+    ctx.sync()
+    assert np.array_equal(_host(buf)[100 + shift:100 + shift + n], oracle.ntt(A, oracle.find_roots(L), L, 1, 1, 1, 1))
+
+
 # 18, 19: two and three blocks a SM
 @pytest.mark.parametrize("L", [1, 2, 3, 8, 9, 10, 15, 16, 17, 18, 19])
 def test_hstep_forms(ctx, oracle, L):
