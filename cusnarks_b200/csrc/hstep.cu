@@ -467,7 +467,7 @@ int cs_ntt_device(cs_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint32_t l
   cudaError_t e = domain_get(ctx, log_n, &dom);
   if (e != cudaSuccess) return fail(ctx, e, "ntt domain");
   const size_t bytes = ((size_t)32 << log_n);
-  if (ntt_overlap(d_in, d_out, log_n)) {
+  if (ntt_overlap(d_in, (size_t)1 << log_n, d_out, (size_t)1 << log_n)) {
     if ((e = ctx->work.reserve(bytes, ctx->stream)) != cudaSuccess) return fail(ctx, e, "ntt scratch");
   }
   NttArgs t;
@@ -496,11 +496,9 @@ int cs_hstep_device(cs_ctx* ctx, int variant, const uint32_t* d_A, const uint32_
   const size_t mb = (size_t)32 << log_m;
   // the reference variant's last transform still reads A and B: where the output lies over one
   // of them they are copied first
-  auto over = [&](const uint32_t* x) {
-    const uintptr_t o = reinterpret_cast<uintptr_t>(d_out), a = reinterpret_cast<uintptr_t>(x);
-    return a < o + 2 * mb && o < a + mb;
-  };
-  const bool copy = variant == CS_HSTEP_REFERENCE && (over(d_A) || over(d_B));
+  const size_t m = (size_t)1 << log_m;
+  const bool copy = variant == CS_HSTEP_REFERENCE &&
+                    (ntt_overlap(d_A, m, d_out, 2 * m) || ntt_overlap(d_B, m, d_out, 2 * m));
   if ((e = ctx->work.reserve((variant == CS_HSTEP_COSET || copy ? 6 : 4) * mb, ctx->stream)) != cudaSuccess)
     return fail(ctx, e, "hstep scratch");
   uint32_t* scr = static_cast<uint32_t*>(ctx->work.ptr);

@@ -259,9 +259,10 @@ cudaError_t ntt_run(const NttArgs& a, cudaStream_t st) {
   uint32_t* work = a.out;
   if (np > 1) {
     // the first pass must not write where other blocks still read
+    const size_t n = (size_t)1 << L, n_in = a.load == NttLoad::kInterleaved ? n / 2 : n;
     bool over = false;
     for (uint32_t z = 0; z < a.count; z++)
-      for (uint32_t y = 0; y < a.count; y++) over |= ntt_overlap(a.in[z], a.out + y * a.out_step, L);
+      for (uint32_t y = 0; y < a.count; y++) over |= ntt_overlap(a.in[z], n_in, a.out + y * a.out_step, n);
     if (over) {
       if (!a.tmp) return cudaErrorInvalidValue;
       work = a.tmp;

@@ -46,10 +46,10 @@ struct NttArgs {
 };
 
 cudaError_t ntt_run(const NttArgs& a, cudaStream_t st);
-// Whether two arrays of 2^log_n elements overlap.
-inline bool ntt_overlap(const uint32_t* x, const uint32_t* y, uint32_t log_n) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y), n = (uintptr_t)32 << log_n;
-  return a < b + n && b < a + n;
+// Whether arrays of nx and ny elements overlap.
+inline bool ntt_overlap(const uint32_t* x, size_t nx, const uint32_t* y, size_t ny) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+  return a < b + ny * 32 && b < a + nx * 32;
 }
 
 // W[j] = root^j for j < count (root: one Montgomery element in device memory).

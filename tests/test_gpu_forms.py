@@ -63,13 +63,20 @@ def test_hstep_forms(ctx, oracle, L):
     A, B, C = (oracle.to_mont(random_field(rng, m, 1), 1) for _ in range(3))
     dA, dB, dC = _dev(A), _dev(B), _dev(C)
     both = _dev(np.concatenate([A, B]))  # the output over its own inputs
+    row = _dev(np.concatenate([B, A, np.zeros((2 * m, 8), np.uint32), C, B]))  # next to them
     M, H = _dev(np.zeros((2 * m, 8), np.uint32)), _dev(np.zeros((m, 8), np.uint32))
     ctx.hstep_device(0, dA.data_ptr(), dB.data_ptr(), 0, L, M.data_ptr())
     ctx.hstep_device(1, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), L, H.data_ptr())
     ctx.hstep_device(0, both.data_ptr(), both.data_ptr() + 32 * m, 0, L, both.data_ptr())
+    at = lambda k: row.data_ptr() + 32 * m * k  # noqa: E731
+    ctx.hstep_device(0, at(1), at(0), 0, L, at(2))
+    ctx.sync()
+    side = _host(row)[2 * m:4 * m].copy()
+    ctx.hstep_device(1, at(1), at(0), at(4), L, at(3))
     ctx.sync()
     want = oracle.interpolandmul(A, B, oracle.find_roots(L + 1), L, 2)
     assert np.array_equal(_host(M), want) and np.array_equal(_host(both), want)
+    assert np.array_equal(side, want) and np.array_equal(_host(row)[3 * m:4 * m], oracle.hstep_coset(A, B, C, L))
     assert np.array_equal(_host(H), oracle.hstep_coset(A, B, C, L))
     assert np.array_equal(_host(dA), A) and np.array_equal(_host(dB), B)
 
