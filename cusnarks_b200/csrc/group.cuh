@@ -28,21 +28,20 @@ CSB_DEV Fq select_fq(bool c, const Fq& a, const Fq& b) {
   return r;
 }
 
-// Equal or opposite points (rare): one lane, canonical arithmetic.  qx, q2: q's first two coordinates
-// and the other two, or x and y where it is affine; read where they lie, 16 bytes at a time.
+// Equal or opposite points (rare): one lane, canonical arithmetic.  Both points are read 16 bytes
+// at a time.
 template <class F>
-__device__ __noinline__ void group_add_slow(const uint32_t* p, const uint32_t* qx, const uint32_t* q2, bool q_affine,
-                                            bool neg, uint32_t* out) {
-  constexpr int FW = FieldWords<F>::value, C = FW / 8;  // coordinates of Fq an element
+__device__ __noinline__ void group_add_slow(const uint32_t* p, const uint32_t* q, bool q_affine, bool neg,
+                                            uint32_t* out) {
+  constexpr int FW = FieldWords<F>::value;
   XYZZ<F> a, b = XYZZ<F>::from_affine(Affine<F>{F::zero(), F::one()});
   uint32_t* aw = reinterpret_cast<uint32_t*>(&a);
   uint32_t* bw = reinterpret_cast<uint32_t*>(&b);
-  const int head = q_affine ? C : 2 * C, have = q_affine ? 2 * C : 4 * C;
-  for (int k = 0; k < 4 * C; k++) {
+  for (int k = 0; k < FW / 2; k++) {  // coordinates of Fq
     Fq x = lds_fq(p + 8 * k).canon();
     for (int i = 0; i < 8; i++) aw[8 * k + i] = x.v[i];
-    if (k >= have) continue;
-    x = lds_fq(k < head ? qx + 8 * k : q2 + 8 * (k - head)).canon();
+    if (q_affine && k >= FW / 4) continue;
+    x = lds_fq(q + 8 * k).canon();
     for (int i = 0; i < 8; i++) bw[8 * k + i] = x.v[i];
   }
   if (neg) b.Y = b.Y.neg();
@@ -130,7 +129,7 @@ struct Group {
     const Fq s1 = val(j == 0 ? 0 : 1, j == 0 ? 2 : 3, a);
     if (__any_sync(0xffffffffu, same)) {
       __syncwarp();  // a vote orders no memory accesses: s1 has been read before level 1 is written over
-      if (same && l == 0) group_add_slow<F>(p, q, q + 16 * C, false, false, scr);
+      if (same && l == 0) group_add_slow<F>(p, q, false, false, scr);
     }
     finish(dst, p, inf1, inf2, same, live, pr, s1, q, q + 16 * C, false, false);
   }
@@ -157,7 +156,11 @@ struct Group {
     // level 4: Y1 PPP, R (Q - X3), ZZZ1 PPP
     const Fq s1 = lds_fq(at(p, j == 0 ? 1 : 3, a));
     // level 1 of the scratch was last read before level 2's barriers
-    if (__any_sync(0xffffffffu, same) && same && l == 0) group_add_slow<F>(p, qx, qy, true, neg, scr);
+    if (__any_sync(0xffffffffu, same) && same && l == 0) {
+      __align__(16) uint32_t q[PW / 2];  // read as uint4
+      for (int i = 0; i < PW / 4; i++) { q[i] = qx[i]; q[PW / 4 + i] = qy[i]; }
+      group_add_slow<F>(p, q, true, neg, scr);
+    }
     finish(dst, p, inf1, false, same, live, pr, s1, qx, qy, true, neg);
   }
 

@@ -53,6 +53,17 @@ def test_outputs_written_before_the_last_input_are_early_clobbered(name):
             assert written >= last_input or "&" in constraint, f"{name}:{line}: operand {k}"
 
 
+def test_local_points_read_16_bytes_at_a_time_are_aligned():
+    """lds_fq reads uint4: an array on the stack that goes to it, or to the out-of-line addition that
+    calls it, has no such alignment of itself."""
+    text = open(os.path.join(CSRC, "group.cuh")).read()
+    arrays = re.findall(r"^(.*)\buint32_t (\w+)\[[^\]]+\];", text, re.M)
+    assert arrays
+    for before, name in arrays:
+        if "__align__(16)" not in before:
+            assert not re.search(r"\b(?:lds_fq|group_add_slow<F>)\([^;]*\b%s\b" % name, text), name
+
+
 def test_statements_are_found():
     n = sum(len(list(_statements(os.path.join(CSRC, f)))) for f in FILES)
     assert n >= 10
